@@ -3,7 +3,7 @@
 // The search replaces the inline core of the reference drivers
 // (src/TranRotaConfSearchNoMini.cu:156-464): the receptor spectra are computed once at context
 // creation and stay resident; a search is cut into waves of rotations, each wave running the
-// five kernels of search_kernels.cu back to back on one stream. Only the per-rotation minimum
+// five kernels of search_kernels.cu and its x pass back to back on one stream. Only the per-rotation minimum
 // energy and best translation leave the device.
 #include <cuda_runtime.h>
 
@@ -165,8 +165,7 @@ namespace {
 bool supported_n(int n) { return n == 32 || n == 64 || n == 96 || n == 128; }
 
 // Times the x pass (the dominant kernel) on the search's first wave under each candidate
-// configuration -- column tile and rotations per CTA for the FP32 form, rotations per CTA for
-// the tensor-core form -- and keeps the fastest for this ligand box. The candidates all compute
+// configuration (rotations per CTA) and keeps the fastest for this ligand box. The candidates all compute
 // the same numbers (deterministic kernels), so the timing runs leave no trace in the results.
 int autotune_xpass(cdk_ctx* c, WaveArgs a, const RotDesc* d_rots, long nRot, int wave, bool tc,
                    cudaStream_t s) {
@@ -181,11 +180,7 @@ int autotune_xpass(cdk_ctx* c, WaveArgs a, const RotDesc* d_rots, long nRot, int
   } else if (tc) {
     for (int ch : {32, 64, 128, 256}) cands.push_back({a.col_tile, ch});
   } else {
-    for (int ct : (c->n <= 64 ? std::vector<int>{16, 8} : std::vector<int>{8}))
-      for (int ch : {16, 32, 64}) {
-        if (xpass2_smem_bytes(c->n, c->K, ct) > 227 * 1024) continue;
-        cands.push_back({ct, ch});
-      }
+    for (int ch : {16, 32, 64}) cands.push_back({a.col_tile, ch});
   }
   cudaEvent_t e0, e1;
   CDK_CUDA(cudaEventCreate(&e0));
@@ -390,7 +385,7 @@ int run_waves(cdk_ctx* c, const float* d_coor, const AtomParam* d_params, const 
   a.range_err = reinterpret_cast<int*>(c->d_misc + 4);
   // the shared-memory streamed x pass writes B in plane groups (whole sectors per store)
   a.bgroup = rows ? stream_bgroup() : 1;
-  a.col_tile = c->opts.col_tile > 0 ? c->opts.col_tile : pick_col_tile(n, K);
+  a.col_tile = c->opts.col_tile > 0 ? c->opts.col_tile : kXpassCols;
   a.kyof = (c->opts.reserved[1] & 1) ? nullptr : c->d_kyof;  // reserved[1] bit 0: FFT planes
   // bit 1: block-stage yz kernel at every n; bit 2: octet yz kernel at every n
   a.yz_block_stages = (c->opts.reserved[1] & 2) ? 1 : (c->opts.reserved[1] & 4) ? 2 : 0;
@@ -403,9 +398,8 @@ int run_waves(cdk_ctx* c, const float* d_coor, const AtomParam* d_params, const 
     set_error("ligand box too large for the tensor-core x pass at this grid size and K");
     return CDK_ERR_UNSUPPORTED;
   }
-  if (xpass2_smem_bytes(n, K, a.col_tile) > 227 * 1024 ||
-      (n <= 64 && a.col_tile != 8 && a.col_tile != 16) || (n > 64 && a.col_tile != 8)) {
-    set_error("column tile must be 8 or 16 (n <= 64) or 8 (n > 64) and fit shared memory");
+  if (!xpass_col_tile_ok(n, a.col_tile)) {
+    set_error("column tile must be 8 or 16 (n <= 64) or 8 (n > 64)");
     return CDK_ERR_INVALID;
   }
   CDK_CUDA(cudaMemsetAsync(c->d_misc + 2, 0, 3 * sizeof(unsigned int), s));
@@ -499,7 +493,7 @@ int run_waves(cdk_ctx* c, const float* d_coor, const AtomParam* d_params, const 
   c->stats[4] = (double)Lb;
   c->stats[5] = (double)wave;
   c->stats[13] = hankel ? (double)hp.cols : streamed ? 4.0 : (double)a.col_tile;
-  c->stats[14] = rows || umma ? 128.0 : (double)(a.chunk > 0 ? a.chunk : (tc ? 64 : 32));
+  c->stats[14] = rows || umma ? 128.0 : tc ? (double)(a.chunk > 0 ? a.chunk : 64) : (double)xpass_rotations_per_cta(a);
   c->stats[16] = hankel ? (f16 ? 7.0 : 6.0) : streamed ? (f16 ? 5.0 : 3.0) : umma ? 2.0 : tc ? 1.0 : 0.0;
   c->stats[15] = (double)(c->gkey_seen);
   return CDK_OK;
@@ -819,7 +813,7 @@ int cdk_ctx_create(int nx, int ny, int nz, float spacing, int K, const float* gr
   float2* scratch = nullptr;
   CTX_CUDA(cudaMalloc(&scratch, sizeof(float2) * K * n * ncol));
   cudaError_t e = launch_receptor_fft(n, K, c->d_grids, scratch, c->d_phat, c->d_tw,
-                                      pick_col_tile(n, 1), c->stream);
+                                      n <= 64 ? 16 : 8, c->stream);
   if (e == cudaSuccess && c->opts.form != CDK_FORM_FP32) {
     e = cudaMalloc(&c->d_ptilde, sizeof(float2) * K * n * ncol);
     if (e == cudaSuccess) e = launch_ptilde(n, K, scratch, c->d_ptilde, c->stream);

@@ -171,9 +171,12 @@ cudaError_t launch_finalize_server(const WaveArgs& a, float* ebase, int* ibase, 
 // Dense forward transform of K receptor grids [K][n][n][n] -> phat [n][K][ncol].
 cudaError_t launch_receptor_fft(int n, int K, const float* grids, float2* scratch,
                                 float2* phat, const float2* tw, int col_tile, cudaStream_t s);
-// Shared memory per CTA of the FP32 x pass for given n, K, column tile.
-size_t xpass2_smem_bytes(int n, int K, int col_tile);
-int pick_col_tile(int n, int K);
+// Column tiles opts.col_tile may name (8, or 16 at n <= 64); the FP32 x pass runs 8 columns per CTA
+// whichever is named, with the same results.
+bool xpass_col_tile_ok(int n, int col_tile);
+constexpr int kXpassCols = 8;
+// rotations per CTA of the FP32 x pass for this wave
+int xpass_rotations_per_cta(const WaveArgs& a);
 // Dense FillLigandGrid on the GPU.
 cudaError_t launch_fill_dense(int nQ, int nAtom, const float* coors, const float* mincoors,
                               const AtomParam* params, int nVdwUsed, int X, int Y, int Z,

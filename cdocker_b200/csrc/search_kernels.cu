@@ -6,7 +6,7 @@
 //   spread_yz     per (rotation, channel, x plane): spread the atoms that touch the plane
 //                 into shared memory (trilinear weights in FillLigandGrid's arithmetic), then
 //                 the 2-D real-to-complex FFT over (y,z) -> A      (src/FillLigandGrid.cpp)
-//   xpass         per spectral column tile: FFT along x of every channel, the conjugate
+//   xpass         (fp32_xpass.cu) per spectral column tile: FFT along x of every channel, the conjugate
 //                 product with the resident receptor spectra summed over channels, and the
 //                 inverse FFT along x, keeping only the translation window -> B
 //                                                       (src/kernel.cu ConjMult + SumGrids)
@@ -632,148 +632,6 @@ __global__ void __launch_bounds__(256, kPlaneColsPerThread == 1 ? 5 : 4) k_sprea
 #pragma unroll
       for (int u = 0; u < CPT; ++u)
         plane_chunk_write<N, LOP>(a, r, k, jc, x0, xlo, xhi, cb + u * (NCOL / CPT), ax[u], ay[u]);
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------------------
-// x pass for two-stage plans (N = R0*R1), fused stage by stage; CT spectral columns per CTA:
-//   phase A  first forward stage straight from A in global memory (only the x planes a
-//            channel touches are read; the rest are known zeros), two channels per round;
-//            the next round's loads are issued before this round's phase B to hide latency
-//   phase B  second forward stage + conj(L_k) * P_k accumulated in registers over all
-//            channels (receptor tile resident in shared memory for the CTA's rotations)
-//   combine  pair sum through one shuffle, first inverse stage
-//   phase C  last inverse stage, written straight to B for x inside the window
-template <int N, int CT>
-__global__ void __launch_bounds__(256, 2) k_xpass2(WaveArgs a, int rot_per_cta) {
-  constexpr int NZH = N / 2 + 1;
-  constexpr int NCOL = N * NZH;
-  constexpr int R0 = FFTPlan<N>::R0, R1 = FFTPlan<N>::R1, M1 = N / R0;
-  constexpr int NA = 2 * CT * M1;  // phase-A items
-  constexpr int NB = 2 * CT * R0;  // phase-B items
-  static_assert(FFTPlan<N>::NS == 2, "two-stage plans only");
-  static_assert(NA <= 256 && NB <= 256, "one item per thread");
-  static_assert(NCOL % CT == 0, "column tiles must divide the half spectrum");
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int K = a.K;
-  float2* tw = reinterpret_cast<float2*>(smem_raw);
-  int* s_ch = reinterpret_cast<int*>(tw + N);               // [KMAX] channel ids, [KMAX] count
-  short* s_rng = reinterpret_cast<short*>(s_ch + 2 * KMAX);  // [KMAX][2] x range per slot
-  float2* Ps = reinterpret_cast<float2*>(s_rng + 4 * KMAX);  // [N][K][CT]
-  float2* Wb = Ps + (size_t)N * K * CT;                      // [N][2][CT]
-  float2* S = Wb + (size_t)N * 2 * CT;                       // [N][CT]
-  const int c0 = blockIdx.x * CT;
-  const int tid = threadIdx.x;
-  for (int i = tid; i < N; i += 256) tw[i] = a.tw[i];
-  for (int i = tid; i < N * K * CT; i += 256) {
-    const int c = i % CT, t = i / CT;  // t = pos*K + k
-    Ps[i] = a.phat[(size_t)t * NCOL + c0 + c];
-  }
-  // per-thread roles
-  const int a_c = tid % CT, a_half = (tid / CT) & 1, a_np = tid / (2 * CT);
-  const int b_half = tid & 1, b_c = (tid >> 1) % CT, b_b = (tid >> 1) / CT;
-  const int r_begin = blockIdx.y * rot_per_cta;
-  const int r_end = min(a.nrot, r_begin + rot_per_cta);
-  for (int r = r_begin; r < r_end; ++r) {
-    const RotRec* rec = a.rec + r;
-    if (!rec->valid) continue;
-    __syncthreads();  // previous rotation is done with s_ch / Wb / S
-    if (tid == 0) {
-      int nk = 0;
-      for (int k = 0; k < K; ++k)
-        if (rec->xlo[k] <= rec->xhi[k]) {
-          s_rng[2 * nk] = rec->xlo[k];
-          s_rng[2 * nk + 1] = rec->xhi[k];
-          s_ch[nk++] = k;
-        }
-      s_ch[KMAX] = nk;
-    }
-    __syncthreads();
-    const int nk = s_ch[KMAX];
-    const float2* Ar = a.A + ((size_t)r * K) * a.Lb * NCOL + c0 + a_c;
-    // raw loads of one round (channels kk0, kk0+1) for this thread's phase-A item
-    auto load_round = [&](int kk0, float2* v) {
-      const int kk = kk0 + a_half;
-      if (tid < NA && kk < nk) {
-        const int k = s_ch[kk];
-        const int lo = s_rng[2 * kk], hi = s_rng[2 * kk + 1];
-        const float2* src = Ar + (size_t)k * a.Lb * NCOL;
-#pragma unroll
-        for (int j = 0; j < R0; ++j) {
-          const int x = a_np + j * M1;
-          v[j] = (x >= lo && x <= hi) ? src[(size_t)x * NCOL] : make_float2(0.f, 0.f);
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < R0; ++j) v[j] = make_float2(0.f, 0.f);
-      }
-    };
-    float2 acc[R1];
-#pragma unroll
-    for (int j = 0; j < R1; ++j) acc[j] = make_float2(0.f, 0.f);
-    float2 va[R0];
-    load_round(0, va);
-    for (int k0 = 0; k0 < nk; k0 += 2) {
-      // phase A: first forward stage into Wb
-      if (tid < NA) {
-        Radix<R0, -1>::run(va);
-#pragma unroll
-        for (int q = 1; q < R0; ++q) va[q] = c_mul(va[q], tw[a_np * q]);
-#pragma unroll
-        for (int q = 0; q < R0; ++q) Wb[((a_np + q * M1) * 2 + a_half) * CT + a_c] = va[q];
-      }
-      __syncthreads();
-      if (k0 + 2 < nk) load_round(k0 + 2, va);  // in flight during phase B
-      // phase B: second forward stage and the conjugate product, accumulated
-      const int kk = k0 + b_half;
-      if (tid < NB && kk < nk) {
-        const int k = s_ch[kk];
-        float2 v[R1];
-#pragma unroll
-        for (int j = 0; j < R1; ++j) v[j] = Wb[((b_b * R1 + j) * 2 + b_half) * CT + b_c];
-        Radix<R1, -1>::run(v);
-#pragma unroll
-        for (int q = 0; q < R1; ++q) {
-          const float2 p = Ps[((b_b * R1 + q) * K + k) * CT + b_c];
-          acc[q].x += v[q].x * p.x + v[q].y * p.y;
-          acc[q].y += v[q].x * p.y - v[q].y * p.x;
-        }
-      }
-      __syncthreads();
-    }
-    // combine the pair (lanes tid, tid^1), first inverse stage, into S
-    if (tid < ((NB + 31) & ~31)) {
-      float2 v[R1];
-#pragma unroll
-      for (int j = 0; j < R1; ++j) {
-        v[j].x = acc[j].x + __shfl_xor_sync(0xffffffffu, acc[j].x, 1);
-        v[j].y = acc[j].y + __shfl_xor_sync(0xffffffffu, acc[j].y, 1);
-      }
-      if (tid < NB && b_half == 0) {
-        Radix<R1, +1>::run(v);
-#pragma unroll
-        for (int j = 0; j < R1; ++j) S[(b_b * R1 + j) * CT + b_c] = v[j];
-      }
-    }
-    __syncthreads();
-    // phase C: last inverse stage, window rows only
-    const int Wx = rec->W[0];
-    if (tid < CT * M1) {
-      const int c = tid % CT, np = tid / CT;
-      float2 v[R0];
-#pragma unroll
-      for (int q = 0; q < R0; ++q) {
-        v[q] = S[(np + q * M1) * CT + c];
-        if (q > 0) v[q] = c_mulc(v[q], tw[np * q]);
-      }
-      Radix<R0, +1>::run(v);
-      float2* dst = a.B + (size_t)r * N * NCOL + c0 + c;
-#pragma unroll
-      for (int j = 0; j < R0; ++j) {
-        const int x = np + j * M1;
-        if (x < Wx) dst[(size_t)x * NCOL] = v[j];
-      }
     }
   }
 }
@@ -1538,30 +1396,6 @@ cudaError_t launch_yz_inv_t(const WaveArgs& a, cudaStream_t s) {
 }
 
 template <int N>
-cudaError_t launch_xpass_t(const WaveArgs& a, cudaStream_t s) {
-  constexpr int NCOL = N * (N / 2 + 1);
-  static_assert(FFTPlan<N>::NS == 2, "the x pass runs two-stage radix plans");
-  // fixed 16-column tiles; chunks of up to 32 rotations per CTA keep the receptor tile
-  // reused while giving the scheduler many CTAs per SM slot
-  constexpr int CT = 16;
-  if (a.col_tile != CT && a.col_tile != 8) return cudaErrorInvalidValue;
-  if (N > 64 && a.col_tile != 8) return cudaErrorInvalidValue;
-  const size_t sm = xpass2_smem_bytes(N, a.K, a.col_tile);
-  const int per = a.chunk > 0 ? a.chunk : 32;
-  const int chunks = (a.nrot + per - 1) / per;
-  if (N <= 64 && a.col_tile == CT) {
-    cudaError_t e = cudaFuncSetAttribute(k_xpass2<N, (N <= 64 ? 16 : 8)>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-    k_xpass2<N, (N <= 64 ? 16 : 8)><<<dim3(NCOL / (N <= 64 ? 16 : 8), chunks), 256, sm, s>>>(a, per);
-  } else {
-    cudaError_t e = cudaFuncSetAttribute(k_xpass2<N, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-    k_xpass2<N, 8><<<dim3(NCOL / 8, chunks), 256, sm, s>>>(a, per);
-  }
-  return cudaGetLastError();
-}
-
-template <int N>
 cudaError_t launch_receptor_t(int K, const float* grids, float2* scratch, float2* phat,
                               const float2* tw, int ct, cudaStream_t s) {
   const size_t sm = plane_smem<N>();
@@ -1705,17 +1539,6 @@ int fft_position(int n, int k) {
   }
 }
 
-size_t xpass2_smem_bytes(int n, int K, int col_tile) {
-  return sizeof(float2) * n + sizeof(int) * 2 * KMAX + sizeof(short) * 4 * KMAX +
-         sizeof(float2) * (size_t)n * col_tile * (K + 2 + 1);
-}
-
-int pick_col_tile(int n, int K) {
-  // 16 columns when the buffers stay within ~110 KB of shared memory (two CTAs per SM), else 8
-  if ((n == 32 || n == 64) && xpass2_smem_bytes(n, K, 16) <= 110 * 1024) return 16;
-  return 8;
-}
-
 #define CDK_DISPATCH_N(n, fn, ...)                 \
   switch (n) {                                     \
     case 32: return fn<32>(__VA_ARGS__);           \
@@ -1766,9 +1589,6 @@ cudaError_t launch_spread_yz(const WaveArgs& a, cudaStream_t s) {
 bool direct_planes(const WaveArgs& a) {
   const int cap = a.atom_cap > 0 ? a.atom_cap : a.max_atoms;
   return a.kyof != nullptr && cap <= kDirectMaxAtoms;
-}
-cudaError_t launch_xpass(const WaveArgs& a, cudaStream_t s) {
-  CDK_DISPATCH_N(a.n, launch_xpass_t, a, s);
 }
 cudaError_t launch_yz_inv_argmin(const WaveArgs& a, cudaStream_t s) {
   CDK_DISPATCH_N(a.n, launch_yz_inv_t, a, s);

@@ -328,7 +328,7 @@ void worker_loop(cdk_server* s) {
   a.tw = s->v.tw;
   a.work = reinterpret_cast<unsigned long long*>(s->d_misc + 32);
   for (int k = 0; k < KMAX; ++k) a.lscale[k] = s->v.lscale[k];
-  a.col_tile = s->v.col_tile_opt > 0 ? s->v.col_tile_opt : pick_col_tile(n, K);
+  a.col_tile = s->v.col_tile_opt > 0 ? s->v.col_tile_opt : kXpassCols;
   a.kyof = s->v.kyof;
   a.minE = nullptr;
   a.idx = nullptr;

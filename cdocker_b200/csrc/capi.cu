@@ -459,10 +459,12 @@ int run_waves(cdk_ctx* c, const float* d_coor, const AtomParam* d_params, const 
   if (hankel && c->tuned_hx_Lb == Lb && c->tuned_hx_cols > 0)
     hankel_plan(n, K, Lb, f16form, c->tuned_hx_cols, &hp, c->tuned_hx_nb, c->tuned_hx_ks);
   if (hankel) hankel_b_layout(hp, a);
+  else if (!tc && a.yz_block_stages == 0) a.bpairs = 2;  // the FP32 x pass writes plane pairs
   if (c->opts.reserved[2]) c->tuned_any_Lb = Lb;
   for (long r0 = 0; r0 < nRot; r0 += wave) {
     a.nrot = (int)std::min<long>(wave, nRot - r0);
     a.rots = order + r0;
+    a.key_slots = a.bpairs ? yz_pairs_key_slots(a) : 0;
     cudaEvent_t* ev = prof ? &c->kev[(size_t)waves * (kLaunchesPerWave + 1)] : nullptr;
     if (prof) CDK_CUDA(cudaEventRecordWithFlags(ev[0], s, evflags));
     CDK_CUDA(launch_prep(a, s));

@@ -77,6 +77,10 @@ struct WaveArgs {
   int bgroup;                // 0 or 1: plain B layout; 2, 4, 8: grouped (tensor-core x passes)
   int bcol;                  // 1: the grouped layout keeps single columns (G x 8 B runs), for
                              // x passes that own one column per CTA
+  int bpairs;                // 2: B in plane pairs [nrot][n/2][ncol] of 16 B (re x, re x+1, im x,
+                             // im x+1); 4: in plane quads [nrot][n/4][ncol][2] of the same 16 B
+                             // (bgroup 4, bcol 1); 0: not paired. Read by launch_yz_pairs only
+  int key_slots;             // key pairs per rotation in keys2 (0: one per window plane)
   int yz_block_stages;       // inverse (y,z) kernel: 0 by grid size (block stages at n <= 64,
                              // octets at n >= 96), 1 block stages, 2 octets
   unsigned long long* keys;  // [nrot]
@@ -164,6 +168,10 @@ cudaError_t launch_group_rotations(const RotDesc* rots, const ConfDesc* confs, c
 cudaError_t launch_spread_yz(const WaveArgs& a, cudaStream_t s);
 cudaError_t launch_xpass(const WaveArgs& a, cudaStream_t s);
 cudaError_t launch_yz_inv_argmin(const WaveArgs& a, cudaStream_t s);
+// the inverse (y,z) pass over paired planes (WaveArgs.bpairs), and the key pairs per rotation it
+// writes (WaveArgs.key_slots)
+cudaError_t launch_yz_pairs(const WaveArgs& a, cudaStream_t s);
+int yz_pairs_key_slots(const WaveArgs& a);
 cudaError_t launch_finalize(const WaveArgs& a, cudaStream_t s);
 // Finalize for waves whose rotations belong to different requests: minE goes to
 // ebase[RotDesc.out], the three indices to ibase[RotDesc.pad0 .. +2].

@@ -321,17 +321,28 @@ __device__ __forceinline__ void xp_body(const WaveArgs& a, const XpTwiddles<N>& 
     group_sync();
     const int W0 = rc.W0;
     float2* dst = a.B + (size_t)(r_begin + s * XP_SET + rot) * N * NCOL + c0 + col;
+    // planes np and np + 1 (np even) of each j together: one 16-byte store in the paired layout
 #pragma unroll 1
-    for (int np = QQ; np < R1; np += 4) {
-      float4 e[4];
+    for (int np = 2 * QQ; np < R1; np += 8) {
+      float2 o[2][8];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) e[q] = sh.exch[(np * 4 + q) * 32 + lane];
-      float2 o[8];
-      xp_last<N>(e, tw, np, o);
+      for (int h = 0; h < 2; ++h) {
+        float4 e[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) e[q] = sh.exch[((np + h) * 4 + q) * 32 + lane];
+        xp_last<N>(e, tw, np + h, o[h]);
+      }
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const int x = np + R1 * j;
-        if (x < W0) dst[(size_t)x * NCOL] = o[j];
+        if (a.bpairs) {
+          if (x < W0)
+            *reinterpret_cast<float4*>(dst + (size_t)x * NCOL + c0 + col) =
+                make_float4(o[0][j].x, o[1][j].x, o[0][j].y, o[1][j].y);
+        } else {
+          if (x < W0) dst[(size_t)x * NCOL] = o[0][j];
+          if (x + 1 < W0) dst[(size_t)(x + 1) * NCOL] = o[1][j];
+        }
       }
     }
   }

@@ -661,9 +661,15 @@ __global__ void __launch_bounds__(HX_THREADS, 2)
 #pragma unroll
           for (int i = 0; i < 16; i += 4) {
             const int xp = x0 + i;
-            if (xp < Wr)
-              st_v8(row2 + (size_t)(xp & ~gm) * NCOL + (size_t)c0 * G2 + (xp & gm), re[0][i], im[0][i],
-                    re[0][i + 1], im[0][i + 1], re[0][i + 2], im[0][i + 2], re[0][i + 3], im[0][i + 3]);
+            if (xp < Wr) {
+              float2* run = row2 + (size_t)(xp & ~gm) * NCOL + (size_t)c0 * G2 + (xp & gm);
+              if (a.bpairs)  // two plane pairs: re, re, im, im each
+                st_v8(run, re[0][i], re[0][i + 1], im[0][i], im[0][i + 1], re[0][i + 2], re[0][i + 3], im[0][i + 2],
+                      im[0][i + 3]);
+              else
+                st_v8(run, re[0][i], im[0][i], re[0][i + 1], im[0][i + 1], re[0][i + 2], im[0][i + 2], re[0][i + 3],
+                      im[0][i + 3]);
+            }
           }
         } else if (bcol && G2 == 2) {
           // single-column groups of 2 planes: one 16-byte run per plane pair
@@ -868,13 +874,17 @@ static int hankel_colgroup() {
 void hankel_b_layout(const HankelPlan& p, WaveArgs& a) {
   a.bcol = p.cols == 1 ? 1 : 0;
   a.bgroup = p.cols == 1 ? hankel_colgroup() : stream_bgroup();
+  // plane quads for the paired inverse (y,z) kernel, unless one of the single-plane kernels is asked for
+  a.bpairs = a.bcol && a.bgroup == 4 && a.yz_block_stages == 0 ? 4 : 0;
 }
 
 cudaError_t launch_xpass_hankel(const WaveArgs& a, const float2* pt, const float* f16_scale,
                                 const HankelPlan& p, cudaStream_t s) {
   if (!a.lop || !pt || a.K > KMAX) return cudaErrorInvalidValue;
   // the B layout must be the plan's (the inverse (y,z) pass reads what this pass writes)
-  if ((a.bcol != 0) != (p.cols == 1) || (a.bcol && a.bgroup != 2 && a.bgroup != 4)) return cudaErrorInvalidValue;
+  if ((a.bcol != 0) != (p.cols == 1) || (a.bcol && a.bgroup != 2 && a.bgroup != 4) ||
+      (a.bpairs && (a.bpairs != 4 || !a.bcol || a.bgroup != 4)))
+    return cudaErrorInvalidValue;
   HxScale sc{};
   for (int k = 0; k < a.K; ++k) sc.s[k] = (a.f16 && f16_scale) ? f16_scale[k] : 1.f;
   // the stage plan of every 128-rotation tile (channels, K-steps, largest window); with tiled

@@ -237,6 +237,7 @@ extern "C" int cdk_search_device_noalloc(cdk_ctx* ctx, int nAtom, int nConf,
   a.work = reinterpret_cast<unsigned long long*>(misc + 4);
   a.col_tile = v.col_tile_opt > 0 ? v.col_tile_opt : kXpassCols;
   a.kyof = v.kyof;
+  a.bpairs = 2;
   for (long r0 = 0; r0 < nRot; r0 += wave) {
     a.nrot = (int)std::min<long>(wave, nRot - r0);
     a.rots = rots;

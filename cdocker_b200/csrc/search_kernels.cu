@@ -26,6 +26,7 @@
 
 #include "cdk_internal.h"
 #include "fft.cuh"
+#include "window_keys.cuh"
 
 namespace cdk {
 
@@ -108,15 +109,6 @@ __device__ __forceinline__ int cell_of(float x, float mn, float h) {
 __device__ __forceinline__ double ratio_of(float x, float mn, float h, int i) {
   return __ddiv_rn(__dsub_rn(__dsub_rn((double)x, (double)mn), (double)__fmul_rn((float)i, h)),
                    (double)h);
-}
-
-__device__ __forceinline__ unsigned int order_key(float f) {
-  unsigned int u = __float_as_uint(f);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ float key_to_float(unsigned int k) {
-  unsigned int u = (k & 0x80000000u) ? (k & 0x7fffffffu) : ~k;
-  return __uint_as_float(u);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -667,64 +659,6 @@ inline int b_layout(const WaveArgs& a) {
   return a.bgroup <= 1 ? kBPlain : a.bgroup == 2 ? kBPairs2 : kBAny;
 }
 
-// keep the two smallest keys (b1 < b2) of a stream of distinct keys
-__device__ __forceinline__ void top2_insert(unsigned long long k, unsigned long long& b1, unsigned long long& b2) {
-  // most candidates lose to the current second-smallest on the energy bits alone (one 32-bit
-  // compare); the 64-bit order decides the rest
-  if ((unsigned int)(k >> 32) > (unsigned int)(b2 >> 32)) return;
-  if (k < b1) {
-    b2 = b1;
-    b1 = k;
-  } else if (k < b2) {
-    b2 = k;
-  }
-}
-// merge another pair of two smallest into (b1, b2)
-__device__ __forceinline__ void top2_merge(unsigned long long o1, unsigned long long o2, unsigned long long& b1,
-                                           unsigned long long& b2) {
-  const unsigned long long n1 = o1 < b1 ? o1 : b1;
-  const unsigned long long hi = o1 < b1 ? b1 : o1;
-  const unsigned long long lo2 = o2 < b2 ? o2 : b2;
-  b2 = hi < lo2 ? hi : lo2;
-  b1 = n1;
-}
-
-// Candidate energies e at linear index lin, into a thread's smallest key (b1) or two smallest
-// keys (b1, b2). thr is the float of the largest key kept (+inf while a slot is empty): a value
-// strictly above it (as floats, the same order as the keys) cannot enter and is rejected before
-// its key is built; equal values, NaN and signed zeros take the exact 64-bit key path.
-template <bool TOP2>
-__device__ __forceinline__ void keep_min(float e, unsigned int lin, unsigned long long& b1, unsigned long long& b2,
-                                         float& thr) {
-  if (e > thr) return;
-  const unsigned long long k = ((unsigned long long)order_key(e) << 32) | lin;
-  if constexpr (TOP2) {
-    top2_insert(k, b1, b2);
-    thr = b2 == ~0ull ? INFINITY : key_to_float((unsigned int)(b2 >> 32));
-  } else {
-    if (k < b1) {
-      b1 = k;
-      thr = key_to_float((unsigned int)(k >> 32));
-    }
-  }
-}
-
-// smallest 64-bit key of the warp: redux on the high words, then on the low words of the lanes
-// holding the smallest high word
-__device__ __forceinline__ unsigned long long warp_min_key(unsigned long long k) {
-  const unsigned int hi = __reduce_min_sync(0xffffffffu, (unsigned int)(k >> 32));
-  const unsigned int lo = __reduce_min_sync(0xffffffffu, (unsigned int)(k >> 32) == hi ? (unsigned int)k : 0xffffffffu);
-  return ((unsigned long long)hi << 32) | lo;
-}
-// the warp's two smallest keys from every lane's (b1 < b2) of distinct keys: the smallest b1,
-// then the smallest of (b2 on the lane holding it, b1 elsewhere)
-template <bool TOP2>
-__device__ __forceinline__ void warp_keep_min(unsigned long long& b1, unsigned long long& b2) {
-  const unsigned long long k1 = warp_min_key(b1);
-  if constexpr (TOP2) b2 = warp_min_key(b1 == k1 ? b2 : b1);
-  b1 = k1;
-}
-
 // inverse (y,z) of one (rotation, x in window) plane + min / first argmin; TOP2: also the
 // plane's second-smallest key, for the FP64 near-tie break (WaveArgs.keys2)
 template <int N, bool TOP2, int BL>
@@ -1114,7 +1048,7 @@ __device__ double pose_energy_fp64(const WaveArgs& a, const float* grids, int r,
 }
 
 // FP64 near-tie break of the argmin (precision forms), warp per rotation: the two smallest keys
-// over the rotation's window planes; when the second energy lies within tol * max(|E1|, 1) of
+// over the rotation's key pairs (one per window plane, or WaveArgs.key_slots); when the second energy lies within tol * max(|E1|, 1) of
 // the first, both translations are re-scored in FP64 (pose_energy_fp64) and the lower one is
 // kept -- the smaller linear index (x-major first) on an exact FP64 tie. The reported energy
 // stays the search's own value at the kept translation. work[4] counts re-scored rotations,
@@ -1127,7 +1061,8 @@ __global__ void __launch_bounds__(128) k_tiebreak(WaveArgs a, const float* __res
   if (!rec->valid) return;
   const int n = a.n;
   unsigned long long b1 = ~0ull, b2 = ~0ull;
-  for (int x = lane; x < rec->W[0]; x += 32)
+  const int slots = a.key_slots > 0 ? a.key_slots : rec->W[0];
+  for (int x = lane; x < slots; x += 32)
     top2_merge(a.keys2[((size_t)r * n + x) * 2], a.keys2[((size_t)r * n + x) * 2 + 1], b1, b2);
   for (int o = 16; o > 0; o >>= 1) {
     const unsigned long long o1 = __shfl_xor_sync(0xffffffffu, b1, o);
@@ -1591,6 +1526,7 @@ bool direct_planes(const WaveArgs& a) {
   return a.kyof != nullptr && cap <= kDirectMaxAtoms;
 }
 cudaError_t launch_yz_inv_argmin(const WaveArgs& a, cudaStream_t s) {
+  if (a.bpairs) return launch_yz_pairs(a, s);
   CDK_DISPATCH_N(a.n, launch_yz_inv_t, a, s);
 }
 cudaError_t launch_topk_rescore(const WaveArgs& a, const float* grids, int k, TopPose* out, cudaStream_t s) {

@@ -411,7 +411,9 @@ void worker_loop(cdk_server* s) {
     a.f16 = (tc_wave && f16) ? 1 : 0;
     a.bgroup = tc_wave ? stream_bgroup() : 1;
     a.bcol = 0;
+    a.bpairs = tc_wave ? 0 : 2;  // the FP32 x pass writes plane pairs
     if (tc_wave && !tile_wave) hankel_b_layout(hp, a);
+    a.key_slots = a.bpairs ? yz_pairs_key_slots(a) : 0;
     if (le == cudaSuccess) {
       note(launch_prep(a, s->stream));
       note(launch_spread_yz(a, s->stream));

@@ -349,7 +349,7 @@ int run_waves(cdk_ctx* c, const float* d_coor, const AtomParam* d_params, const 
   const size_t b_keys2 = tiebreak ? align_up((size_t)wave * n * 2 * sizeof(unsigned long long)) : 0;
   const size_t b_A = align_up(rows ? lop_wave_bytes(wave, tiled, lop_per)
                                    : (size_t)wave * K * Lb * ncol * sizeof(float2));
-  const size_t b_B = align_up((size_t)wave * n * ncol * sizeof(float2));
+  const size_t b_B = align_up(b_rotations(wave) * n * ncol * sizeof(float2));
   if (!grow(c->wave, b_rotxyz + b_rec + b_keys + b_A + b_B + b_keys2)) {
     set_error("cudaMalloc of the wave scratch failed (" +
               std::to_string((b_rotxyz + b_rec + b_keys + b_A + b_B + b_keys2) >> 20) + " MiB)");

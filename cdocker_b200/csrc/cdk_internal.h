@@ -78,8 +78,10 @@ struct WaveArgs {
   int bcol;                  // 1: the grouped layout keeps single columns (G x 8 B runs), for
                              // x passes that own one column per CTA
   int bpairs;                // 2: B in plane pairs [nrot][n/2][ncol] of 16 B (re x, re x+1, im x,
-                             // im x+1); 4: in plane quads [nrot][n/4][ncol][2] of the same 16 B
-                             // (bgroup 4, bcol 1); 0: not paired. Read by launch_yz_pairs only
+                             // im x+1); 4: in plane quads [nrot/R][n/4][ncol][R][2] of the same
+                             // 16 B, R = b_quad_rots(n), a rotation's place of R b_quad_slot
+                             // (nrot rounded up to a multiple of R; bgroup 4, bcol 1); 0: not
+                             // paired. Read by launch_yz_pairs only
   int key_slots;             // key pairs per rotation in keys2 (0: one per window plane)
   int yz_block_stages;       // inverse (y,z) kernel: 0 by grid size (block stages at n <= 64,
                              // octets at n >= 96), 1 block stages, 2 octets
@@ -139,6 +141,26 @@ inline bool use_stream_tiles(int variant) { return variant == 3; }
 // (and the driver provides the tensor-map encoder; without it the per-rotation copies run)
 bool tensor_maps_available();
 inline bool hankel_tiled(int reserved5) { return !(reserved5 & 32) && tensor_maps_available(); }
+// Rotations side by side in the plane quads of B. The x pass's store instruction covers 32 rotations,
+// whose planes lie a rotation's B apart: 1.1 MB at 64^3, but 3.6 MB at 96^3 and 8.5 MB at 128^3, a page
+// of their own each. Two rotations per 64-byte run halve the pages and lines of a store (x pass 128^3,
+// 1e5 rotations: 562 -> 390 ms, yz 362 -> 397; 96^3: 215 -> 184, 132 -> 142); at 64^3 the yz pass lost
+// what the x pass gained (46.8 for 48.2 ms, 34.3 for 31.7). Four or more gave the x pass nothing further.
+constexpr int b_quad_rots(int n) { return n >= 96 ? 2 : 1; }
+// rotations a wave's window planes (WaveArgs.B) are allocated for
+inline size_t b_rotations(long nrot) { return (size_t)((nrot + 1) & ~1L); }
+#ifdef __CUDACC__
+// Place of rotation r in its rotation pair: alternating with kz, so that a quarter-warp's four
+// neighbouring columns (64 bytes apart) lie in four different 32-byte bank groups
+__host__ __device__ inline int b_quad_slot(int r, int kz) { return (r ^ (kz >> 1)) & 1; }
+// float4 (plane pair) index in B of the first plane quad of rotation r, column c; the next quads
+// follow n/4-fold at ncol * 2 R float4
+template <int N>
+__host__ __device__ inline size_t b_quad_index(int r, int c) {
+  constexpr int NZH = N / 2 + 1, R = b_quad_rots(N);
+  return ((size_t)(r / R) * (N / 4) * (N * NZH) + c) * (2 * R) + (R == 2 ? b_quad_slot(r, c % NZH) * 2 : 0);
+}
+#endif
 // bytes of a wave's ligand rows (per-rotation bytes times the rotations allocated)
 inline size_t lop_wave_bytes(long nrot, bool tiled, size_t per_rotation) {
   return lop_rotations(nrot, tiled) * per_rotation;

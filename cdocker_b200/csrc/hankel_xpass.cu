@@ -656,19 +656,20 @@ __global__ void __launch_bounds__(HX_THREADS, 2)
           }
         } else if (bcol && G2 >= 4) {
           // single-column groups: float2 of plane xp at (xp - xp % G) NCOL + c G + xp % G; four
-          // planes from xp (a multiple of 4) are one 32-byte run
+          // planes from xp (a multiple of 4) are one 32-byte run (in plane quads of rotation pairs half
+          // of a 64-byte run, whose other half the neighbouring lane writes)
           float2* row2 = reinterpret_cast<float2*>(rowp);
+          float4* quad = reinterpret_cast<float4*>(a.B) + b_quad_index<N>(r0 + rl, c0);
 #pragma unroll
           for (int i = 0; i < 16; i += 4) {
             const int xp = x0 + i;
             if (xp < Wr) {
-              float2* run = row2 + (size_t)(xp & ~gm) * NCOL + (size_t)c0 * G2 + (xp & gm);
               if (a.bpairs)  // two plane pairs: re, re, im, im each
-                st_v8(run, re[0][i], re[0][i + 1], im[0][i], im[0][i + 1], re[0][i + 2], re[0][i + 3], im[0][i + 2],
-                      im[0][i + 3]);
+                st_v8(quad + (size_t)(xp >> 2) * (NCOL * 2 * b_quad_rots(N)), re[0][i], re[0][i + 1], im[0][i], im[0][i + 1], re[0][i + 2],
+                      re[0][i + 3], im[0][i + 2], im[0][i + 3]);
               else
-                st_v8(run, re[0][i], im[0][i], re[0][i + 1], im[0][i + 1], re[0][i + 2], im[0][i + 2], re[0][i + 3],
-                      im[0][i + 3]);
+                st_v8(row2 + (size_t)(xp & ~gm) * NCOL + (size_t)c0 * G2 + (xp & gm), re[0][i], im[0][i], re[0][i + 1],
+                      im[0][i + 1], re[0][i + 2], im[0][i + 2], re[0][i + 3], im[0][i + 3]);
             }
           }
         } else if (bcol && G2 == 2) {

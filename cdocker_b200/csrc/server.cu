@@ -320,7 +320,7 @@ void worker_loop(cdk_server* s) {
   unsigned char* lop_base = reinterpret_cast<unsigned char*>(sc);
   sc += up(std::max((size_t)W * K * Lmax * ncol * sizeof(float2), rows));
   a.B = reinterpret_cast<float2*>(sc);
-  sc += up((size_t)W * n * ncol * sizeof(float2));
+  sc += up(b_rotations(W) * n * ncol * sizeof(float2));
   // precision forms: every window plane's two smallest keys for the FP64 near-tie break, as
   // in a plain search (so results are the same alone and in the mix)
   a.keys2 = s->v.tiebreak ? reinterpret_cast<unsigned long long*>(sc) : nullptr;
@@ -513,7 +513,7 @@ int cdk_server_create(cdk_ctx* ctx, const cdk_server_opts* opts, cdk_server** ou
                                   : 0;
   const size_t scratch = up((size_t)W * s->opts.max_atoms * sizeof(float4)) +
                          up((size_t)W * sizeof(RotRec)) + up((size_t)W * 8) +
-                         up(std::max(planes, rows)) + up((size_t)W * n * ncol * sizeof(float2)) +
+                         up(std::max(planes, rows)) + up(b_rotations(W) * n * ncol * sizeof(float2)) +
                          (s->v.tiebreak ? up((size_t)W * n * 2 * sizeof(unsigned long long)) : 0);
   auto fail = [&](const std::string& m, int code) {
     set_error(m);

@@ -6,8 +6,8 @@
 // packed as one complex line over z, keys of (energy, linear index); results are bit-identical.
 //
 // B holds the two planes' values of a spectral column side by side (re x, re x+1, im x, im x+1: 16
-// bytes), either as plane pairs [n/2][ncol] (FP32 x pass) or as plane quads [n/4][ncol][2] (one-
-// column Hankel x pass, whose stores must fill 32-byte sectors).
+// bytes), either as plane pairs (FP32 x pass) or as plane quads (one-column Hankel x pass, whose
+// stores must fill 32-byte sectors).
 //
 // CTA = a rotation and a part of its plane pairs, looped. An octet of 8 lanes owns a line (a kz
 // column for y, a row pair for z): lane t takes block t in the first stage and the groups np = t,
@@ -106,9 +106,11 @@ __global__ void __launch_bounds__(YzShape<N>::T, YzShape<N>::CTAS) k_yz_pairs(co
     const float2 x = unpk(v.x), y = unpk(v.y);
     *p = make_float4(x.x, x.y, y.x, y.y);
   };
-  constexpr int BS = QUADS ? 2 : 1;  // float4 per column
+  constexpr int BS = QUADS ? 2 * b_quad_rots(N) : 1;  // float4 per column
   const bool has_col = gy < NZH;
-  const float4* src0 = reinterpret_cast<const float4*>(a.B + (size_t)r * N * NCOL) + (ty * R1 * NZH + (has_col ? gy : 0)) * BS;
+  const int c0 = ty * R1 * NZH + (has_col ? gy : 0);  // column of the block's first row
+  const float4* src0 = reinterpret_cast<const float4*>(a.B) +
+                       (QUADS ? b_quad_index<N>(r, c0) : (size_t)r * (N / 2) * NCOL + c0);
   float4* const col = O + (has_col ? gy : 0);
   const int sw = R1 % 8 == 0 ? t : t >> 1;  // swizzle of a line's positions t R1 + m -> t R1 + (m ^ sw)
   const float inv = 1.0f / (float)((double)N * N * N);
@@ -118,7 +120,7 @@ __global__ void __launch_bounds__(YzShape<N>::T, YzShape<N>::CTAS) k_yz_pairs(co
   for (int p = part; p < pairs; p += parts) {
     // y of column gy: first stage (radix R1, no twiddles) over block ty's positions
     if (has_col) {
-      const float4* src = QUADS ? src0 + (size_t)(p >> 1) * (NCOL * 2) + (p & 1) : src0 + (size_t)p * NCOL;
+      const float4* src = QUADS ? src0 + (size_t)(p >> 1) * (NCOL * BS) + (p & 1) : src0 + (size_t)p * NCOL;
       cpair v[R1];
 #pragma unroll
       for (int j = 0; j < R1; ++j) v[j] = ld(src + j * NZH * BS);

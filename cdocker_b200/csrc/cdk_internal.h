@@ -44,6 +44,8 @@ struct RotRec {
   int valid;        // 1 when every window is non-empty
   int err;          // nonzero when the ligand box exceeded the planned box
   int nA;           // atoms
+  int param_off;    // first AtomParam of its ligand (ConfDesc.param_off)
+  int pad[3];
   short xlo[KMAX];  // per channel: first and last x plane touched (xlo > xhi: empty)
   short xhi[KMAX];
   // streamed tensor-core x pass, first record of each 128-rotation tile only: the tile's stage
@@ -120,8 +122,6 @@ struct WaveArgs {
                              //    swizzle; chunks of the tile's stage plan that a valid rotation
                              //    does not touch hold zeros (the plane kernel runs after
                              //    k_tile_plan)
-  int plane_rot_major;       // set by the plane kernel's launcher: grid (nrot, K) instead of
-                             // (K, nrot)
 };
 // rotations per tensor-core tile (the MMA's M), and the bytes of one K-step (128 rows of 32 B)
 // of one column and part in the tiled ligand-row layout

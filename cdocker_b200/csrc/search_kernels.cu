@@ -22,10 +22,11 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include <cstdlib>
+#include <algorithm>
 
 #include "cdk_internal.h"
 #include "fft.cuh"
+#include "pair_fft.cuh"
 #include "window_keys.cuh"
 
 namespace cdk {
@@ -208,6 +209,7 @@ __global__ void __launch_bounds__(128) k_prep(WaveArgs a) {
     rec->valid = (valid && !err) ? 1 : 0;
     rec->err = err;
     rec->nA = nA;
+    rec->param_off = cd.param_off;
     a.keys[r] = ~0ull;
   }
 }
@@ -326,66 +328,31 @@ __global__ void __launch_bounds__(256) k_spread_yz(WaveArgs a) {
 //   A(x, ky, kz) = sum_{atoms a touching x} s_a wx_a(x) Fy_a(ky) Fz_a(kz),
 //   Fy_a(ky) = (1 - ry) w^(yi ky) + ry w^((yi+1) ky),   w = exp(-2 pi i / n)
 // (the same numbers the spread + radix FFT produce, without the float rounding of the plane).
-// CTA per (rotation, channel): per-atom factor tables in shared memory, then every touched
-// plane's n*(n/2+1) outputs, written in the (ky position, kz) order of the FFT path.
-// Atoms are visited in ascending order for every plane: deterministic.
-// One column's 8-plane chunk jc of the plane kernel, written as FP32 planes (A), FP16 rows or
-// split-BF16 rows (lop).
-template <int N, bool LOP>
-__device__ __forceinline__ void plane_chunk_write(const WaveArgs& a, int r, int k, int jc, int x0,
-                                                  int xlo, int xhi, int c, const float* ax,
-                                                  const float* ay) {
+// Per-atom factor tables in shared memory, then every touched plane's n*(n/2+1) outputs, written in
+// the (ky position, kz) order of the FFT path. Atoms are visited in ascending order for every plane:
+// deterministic.
+// What the plane kernel writes: FP32 planes (A), or the tensor-core x pass's ligand rows (lop)
+constexpr int kRowsNone = 0, kRowsF16 = 1, kRowsBf16 = 2;
+
+// One column's 8-plane chunk jc as ligand rows, h: the rows' 16-byte words -- split-FP16: [re, im]
+// of the planes times 2^sigma_k (already in the atoms' x weights; k_prep has checked that the
+// scaled planes stay inside the FP16 range); split-BF16: [hi re, hi im, lo re, lo im]. Untiled: per
+// (rotation, channel) 8 or 16 rows [hi, lo][chunk][re, im] of ncol x 16 B, the tensor-core x
+// pass's K order, in 512 B blocks of (8 rotations x 4 columns) x 16 B.
+template <int N, int ROWS>
+__device__ __forceinline__ void plane_rows_write(const WaveArgs& a, int r, int k, int jc, int c, const uint4* h) {
   constexpr int NCOL = N * (N / 2 + 1);
-  if constexpr (!LOP) {
-#pragma unroll
-    for (int d = 0; d < 8; ++d) {
-      const int x = x0 + d;
-      if (x >= xlo && x <= xhi) a.A[(((size_t)r * a.K + k) * a.Lb + x) * NCOL + c] = make_float2(ax[d], ay[d]);
-    }
-  } else if (a.f16) {
-    // split-FP16 form: FP16 rows of the 8 planes times 2^sigma_k (already in the atoms' x
-    // weights): per (rotation, channel) 8 rows [chunk][re, im] of ncol x 16 B in the same 512 B
-    // blocks (k_prep has checked that the scaled planes stay inside the FP16 range)
-    uint32_t hr[4], hi[4];
-#pragma unroll
-    for (int d = 0; d < 8; d += 2) {
-      const __half2 pr = __floats2half2_rn(ax[d], ax[d + 1]), pi = __floats2half2_rn(ay[d], ay[d + 1]);
-      hr[d / 2] = *reinterpret_cast<const uint32_t*>(&pr);
-      hi[d / 2] = *reinterpret_cast<const uint32_t*>(&pi);
-    }
-    if (a.lop_tiled) {
-      tiled_row_store(a, r, k, jc, c, make_uint4(hr[0], hr[1], hr[2], hr[3]), make_uint4(hi[0], hi[1], hi[2], hi[3]));
-      return;
-    }
-    uint4* dst = reinterpret_cast<uint4*>(a.lop) +
-                 (((size_t)(r >> 3) * a.K + k) * 8 * (NCOL / 4) + (c >> 2)) * 32 + (r & 7) * 4 + (c & 3);
-    constexpr size_t RS = (size_t)(NCOL / 4) * 32;  // one row
-    dst[(jc * 2 + 0) * RS] = make_uint4(hr[0], hr[1], hr[2], hr[3]);
-    dst[(jc * 2 + 1) * RS] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-  } else {
-    // split-BF16 rows of the 8 planes (zero outside [xlo, xhi] by construction): per
-    // (rotation, channel) 16 rows [hi, lo][chunk][re, im] of ncol x 16 B, the tensor-core x
-    // pass's K order, in 512 B blocks of (8 rotations x 4 columns) x 16 B
-    uint32_t rh[4], rl[4], ih[4], il[4];
-#pragma unroll
-    for (int d = 0; d < 8; d += 2) {
-      split_bf16x2(ax[d], ax[d + 1], rh[d / 2], rl[d / 2]);
-      split_bf16x2(ay[d], ay[d + 1], ih[d / 2], il[d / 2]);
-    }
-    if (a.lop_tiled) {
-      const uint4 rows[4] = {make_uint4(rh[0], rh[1], rh[2], rh[3]), make_uint4(ih[0], ih[1], ih[2], ih[3]),
-                             make_uint4(rl[0], rl[1], rl[2], rl[3]), make_uint4(il[0], il[1], il[2], il[3])};
-      tiled_row_store64(a, r, k, jc, c, rows);
-      return;
-    }
-    uint4* dst = reinterpret_cast<uint4*>(a.lop) +
-                 (((size_t)(r >> 3) * a.K + k) * 16 * (NCOL / 4) + (c >> 2)) * 32 + (r & 7) * 4 + (c & 3);
-    constexpr size_t RS = (size_t)(NCOL / 4) * 32;  // one row
-    dst[((0 * 4 + jc) * 2 + 0) * RS] = make_uint4(rh[0], rh[1], rh[2], rh[3]);
-    dst[((0 * 4 + jc) * 2 + 1) * RS] = make_uint4(ih[0], ih[1], ih[2], ih[3]);
-    dst[((1 * 4 + jc) * 2 + 0) * RS] = make_uint4(rl[0], rl[1], rl[2], rl[3]);
-    dst[((1 * 4 + jc) * 2 + 1) * RS] = make_uint4(il[0], il[1], il[2], il[3]);
+  constexpr int PER = ROWS == kRowsF16 ? 8 : 16;
+  if (a.lop_tiled) {
+    if constexpr (ROWS == kRowsF16) tiled_row_store(a, r, k, jc, c, h[0], h[1]);
+    else tiled_row_store64(a, r, k, jc, c, h);
+    return;
   }
+  uint4* dst = reinterpret_cast<uint4*>(a.lop) +
+               (((size_t)(r >> 3) * a.K + k) * PER * (NCOL / 4) + (c >> 2)) * 32 + (r & 7) * 4 + (c & 3);
+  constexpr size_t RS = (size_t)(NCOL / 4) * 32;  // one row
+#pragma unroll
+  for (int i = 0; i < PER / 4; ++i) dst[(((i >> 1) * 4 + jc) * 2 + (i & 1)) * RS] = h[i];
 }
 
 // Tiled rows: zeros for a chunk of the tile's stage plan that this rotation's channel does not
@@ -415,215 +382,251 @@ __device__ __forceinline__ void tile_plan_range(const WaveArgs& a, int r, int k,
     }
 }
 
-// plane kernel CTA order for tiled rows: rotation-major by default; the environment variable
-// CDK_PLANE_ORDER=1 keeps the channel-major order, for measurement
-int plane_rot_major_host() {
-  static const int v = [] {
-    const char* e = std::getenv("CDK_PLANE_ORDER");
-    return (e && std::atoi(e) == 1) ? 0 : 1;
-  }();
-  return v;
-}
-
-constexpr int kPlaneColsPerThread = 2;  // columns per thread in the plane kernel
 constexpr int kDirectMaxAtoms = 96;
+constexpr int kDirectWords = kDirectMaxAtoms / 32;
 
-template <int N, bool LOP>
-__global__ void __launch_bounds__(256, kPlaneColsPerThread == 1 ? 5 : 4) k_spread_yz_direct(WaveArgs a, const int* __restrict__ kyof,
-                                                           int cap) {
-  constexpr int NZH = N / 2 + 1;
-  constexpr int NCOL = N * NZH;
+// Shape of the direct plane kernel: threads per CTA and CTAs per SM asked for (registers), shared
+// memory for ligands of at most cap atoms
+template <int N, int ROWS>
+struct DirectShape {
+  static constexpr int NZH = N / 2 + 1, NCOL = N * NZH;
+  static constexpr int Q = NCOL / 4;  // column quads: c, c + Q, c + 2 Q, c + 3 Q share kz
+  static_assert(NCOL % 4 == 0 && Q % NZH == 0, "a quad's columns share kz");
+  // measured (ms): planes at 64^3, 5,000 rotations: 384 x 2 1.52, 256 x 3 1.65; at 32^3 256 x 3 is the
+  // faster; FP16 rows at 64^3, 1e5 rotations: 256 x 3 27.1, 384 x 2 27.7, 192 x 4 27.4; at 128^3, 4,000:
+  // 384 x 2 5.6, 256 x 3 6.2 (shared memory holds two CTAs); BF16 rows, 64 result words per thread: at
+  // 64^3, 2e4: 192 x 3 9.7, 256 x 2 10.0; at 96^3, 2,000: 2.35 and 2.30; at 128^3, 1,000: 384 x 1 2.5,
+  // 192 x 3 3.0
+  static constexpr bool WIDE = ROWS == kRowsNone ? N >= 64 : ROWS == kRowsF16 ? N >= 96 : N >= 128;
+  static constexpr int T = WIDE ? 384 : ROWS == kRowsBf16 && N <= 64 ? 192 : 256;
+  static constexpr int CTAS = ROWS == kRowsBf16 ? (N == 128 ? 1 : N == 96 ? 2 : 3) : WIDE ? 2 : 3;
+  static size_t smem(int cap) {
+    return sizeof(float2) * (N + (size_t)cap * (N + NZH)) + (4 + 1 + 1) * sizeof(int4) * cap + sizeof(float2) * cap;
+  }
+};
+
+// Bound: DRAM writes and issue slots together. CTA = a rotation (and a part of its items): cells,
+// weights and the separable factors of every atom once, for the atom's vdW channel and the
+// electrostatic one. An item is a chunk of 8 planes of one channel; a warp evaluates 32 column quads
+// of it, plane by plane: the atoms of a plane come from a list in ascending order (an atom is in the
+// lists of its planes xi and xi + 1), so a visit is a fixed sequence of 4 shared loads, 16 scalar
+// FMAs (the four columns' Fy Fz) and 4 packed ones (weight times product into the plane's sums).
+// Before, a CTA per (rotation, channel) walked a chunk's atoms with a switch on each one's plane
+// offset, two columns per thread: 264 k warp instructions per rotation at 64^3, K = 9, 40 atoms,
+// 10 % of them floating point. ms before -> now: FP16 rows 64^3, 1e5 rotations 36 -> 27 (the writes'
+// floor 23), 96^3, 2,107: 3.5 -> 1.9, 128^3, 4,000: 9.0 -> 5.6; BF16 rows 64^3, 2e4: 10.2 -> 9.7 (floor
+// 9.4); planes 64^3, 5,000: 1.77 -> 1.52 (floor 1.35), 128^3, 1,000: 2.25 -> 1.75. Bit-identical.
+template <int N, int ROWS>
+__global__ void __launch_bounds__(DirectShape<N, ROWS>::T, DirectShape<N, ROWS>::CTAS)
+    k_spread_yz_direct(const __grid_constant__ WaveArgs a, const int* __restrict__ kyof, int cap) {
+  using S = DirectShape<N, ROWS>;
+  constexpr int NZH = S::NZH, NCOL = S::NCOL, Q = S::Q, NY = N / 4, T = S::T, NW = T / 32;
+  constexpr bool LOP = ROWS != kRowsNone;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float2* tw = reinterpret_cast<float2*>(smem_raw);            // [N]
-  int4* s_apk = reinterpret_cast<int4*>(tw + N);                // [cap] (x cell, w(xi), w(xi+1), -)
-  float2* Fy = reinterpret_cast<float2*>(s_apk + cap);          // [cap][N/2][2]: ky positions p, p + N/2
-  float2* Fz = Fy + (size_t)cap * N;                            // [cap][NZH]
-  int2* s_yz = reinterpret_cast<int2*>(Fz + (size_t)cap * NZH);  // [cap] y and z cells
-  float2* s_rr = reinterpret_cast<float2*>(s_yz + cap);           // [cap] y and z ratios
-  int* s_atom = reinterpret_cast<int*>(s_rr + cap);               // [cap]
-  __shared__ int s_cnt;
-  __shared__ uint32_t s_cm[N / 8][3];  // per 8-plane chunk: the channel atoms touching it (bit j)
-  // grid (K, nrot), or (nrot, K) for tiled rows: the CTAs in flight then write whole
-  // 128-rotation blocks of one channel together
-  const bool rot_major = LOP && a.plane_rot_major;
-  const int k = rot_major ? blockIdx.y : blockIdx.x, r = rot_major ? blockIdx.x : blockIdx.y;
+  int4* s_cell = reinterpret_cast<int4*>(smem_raw);                // [cap] x, y, z cells, slot
+  float4* s_w = reinterpret_cast<float4*>(s_cell + cap);           // [cap] vdW w(xi), w(xi+1), elec w(xi), w(xi+1)
+  int4* s_list = reinterpret_cast<int4*>(s_w + cap);               // [4 cap] (w, w, Fy offset, Fz offset)
+  float4* Fy = reinterpret_cast<float4*>(s_list + 4 * cap);        // [cap][NY][2]: re, re, im, im of positions
+                                                                   // (p, p + NY) and (p + 2 NY, p + 3 NY)
+  float2* Fz = reinterpret_cast<float2*>(Fy + (size_t)cap * NY * 2);  // [cap][NZH]
+  float2* tw = Fz + (size_t)cap * NZH;                             // [N]
+  float2* s_rr = tw + N;                                           // [cap] y and z ratios
+  __shared__ uint32_t s_plane[N][kDirectWords];   // atoms with a cell on the plane (bit j)
+  __shared__ uint32_t s_chan[KMAX][kDirectWords];  // atoms of the channel
+  __shared__ uint32_t s_run[KMAX][N];             // list entries of (channel, plane): first | count << 16
+  __shared__ uint16_t s_item[KMAX * (N / 8)];     // channel | chunk << 4 | untouched << 8
+  __shared__ int s_nitems;
+  const int r = blockIdx.y;
   const RotRec* rec = a.rec + r;
   if (!rec->valid) return;
-  const int xlo = rec->xlo[k], xhi = rec->xhi[k];
-  const int tid = threadIdx.x, nthr = blockDim.x;
-  // tiled rows: the chunks of the tile's plan outside this rotation's own range get zeros
-  int zlo = 15, zhi = -1;
-  if (LOP && a.lop_tiled) tile_plan_range(a, r, k, zlo, zhi);
-  if (xlo > xhi) {
-    for (int q = zlo; q <= zhi; ++q)
-      for (int c = tid; c < NCOL; c += nthr) tiled_zero_chunk(a, r, k, q, c);
-    return;
-  }
-  for (int i = tid; i < N; i += nthr) tw[i] = a.tw[i];
-  const RotDesc rd = a.rots[r];
-  const ConfDesc cd = a.confs[rd.conf];
-  const AtomParam* prm = a.params + cd.param_off;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int K = a.K, elec = K - 1;
+  const int na = min(rec->nA, cap);
+  const AtomParam* prm = a.params + rec->param_off;
   const float mn0 = rec->mn[0], mn1 = rec->mn[1], mn2 = rec->mn[2];
   const float h = a.spacing;
-  const bool elec = (k == a.K - 1);
-  const int nA = rec->nA;
-  // channel atoms in ascending order (warp 0, ballot compaction)
-  if (tid < 32) {
-    int cnt = 0;
-    for (int base = 0; base < nA; base += 32) {
-      const int i = base + tid;
-      const bool in = i < nA && (elec || prm[i].slot == k);
-      const unsigned int m = __ballot_sync(0xffffffffu, in);
-      if (in) s_atom[cnt + __popc(m & ((1u << tid) - 1))] = i;
-      cnt += __popc(m);
-    }
-    if (tid == 0) s_cnt = cnt;
-  }
-  __syncthreads();
-  const int na = s_cnt;
+  for (int i = tid; i < N; i += T) tw[i] = a.tw[i];
+  // per atom: cells, ratios and x weights (FillLigandGrid's double arithmetic, once per atom);
   // split-FP16 rows carry 2^sigma_k: a power of two, folded exactly into the x weights (every
   // product and sum below then scales exactly, outside under- and overflow)
-  const float wsc = (LOP && a.f16) ? a.lscale[k] : 1.f;
-  // per atom: cells, ratios and x weights (FillLigandGrid's double arithmetic, once per atom)
-  for (int j = tid; j < na; j += nthr) {
-    const int at = s_atom[j];
-    const float4 p = a.rot_xyz[(size_t)r * a.max_atoms + at];
+  for (int j = tid; j < na; j += T) {
+    const AtomParam ap = prm[j];
+    const float4 p = a.rot_xyz[(size_t)r * a.max_atoms + j];
     const int xi = cell_of(p.x, mn0, h), yi = cell_of(p.y, mn1, h), zi = cell_of(p.z, mn2, h);
     const double xr = ratio_of(p.x, mn0, h, xi);
-    const double sc = elec ? (double)prm[at].charge : (double)prm[at].w_vdw;
-    s_apk[j] = make_int4(xi, __float_as_int(__fmul_rn((float)(sc * (1.0 - xr)), wsc)),
-                         __float_as_int((xi + 1 < N) ? __fmul_rn((float)(sc * xr), wsc) : 0.f), 0);
-    s_yz[j] = make_int2(yi, zi);
+    const bool vdw = ap.slot >= 0 && ap.slot < elec;
+    const float sv = ROWS == kRowsF16 && vdw ? a.lscale[vdw ? ap.slot : 0] : 1.f, se = ROWS == kRowsF16 ? a.lscale[elec] : 1.f;
+    const double wv = (double)ap.w_vdw, we = (double)ap.charge;
+    const bool next = xi + 1 < N;
+    s_cell[j] = make_int4(xi, yi, zi, vdw ? ap.slot : -1);
+    s_w[j] = make_float4(__fmul_rn((float)(wv * (1.0 - xr)), sv), next ? __fmul_rn((float)(wv * xr), sv) : 0.f,
+                         __fmul_rn((float)(we * (1.0 - xr)), se), next ? __fmul_rn((float)(we * xr), se) : 0.f);
     s_rr[j] = make_float2((float)ratio_of(p.y, mn1, h, yi), (float)ratio_of(p.z, mn2, h, zi));
+  }
+  // items: the touched chunks of every channel and, for tiled rows, the chunks of the tile's stage
+  // plan that this rotation does not touch (zeros)
+  const int chunks = (rec->xhi[elec] >> 3) + 1;  // elec: every atom; planes < n, so <= n / 8
+  if (warp == 0) {
+    int lo = 1, hi = 0, own_lo = 1, own_hi = 0;
+    if (lane < K) {
+      const int xlo = rec->xlo[lane], xhi = rec->xhi[lane];
+      if (xlo <= xhi) own_lo = lo = xlo >> 3, own_hi = hi = xhi >> 3;
+      if (LOP && a.lop_tiled) tile_plan_range(a, r, lane, lo, hi);
+    }
+    const int cnt = max(0, hi - lo + 1);
+    int end = cnt;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, end, o);
+      if (lane >= o) end += v;
+    }
+    for (int q = lo; q <= hi; ++q)
+      s_item[end - cnt + q - lo] = (uint16_t)(lane | q << 4 | (q < own_lo || q > own_hi ? 256 : 0));
+    if (lane == 31) s_nitems = end;
   }
   __syncthreads();
   // factor tables
-  for (int i = tid; i < na * (N + NZH); i += nthr) {
+  for (int i = tid; i < na * (N + NZH); i += T) {
     const int j = i / (N + NZH), f = i - j * (N + NZH);
     if (f < N) {
-      const int yi = s_yz[j].x;
+      const int yi = s_cell[j].y;
       const float ry = s_rr[j].x;
       const int ky = kyof[f];  // natural frequency of position f
       const float2 w0 = tw[(yi * ky) % N], w1 = tw[((yi + 1) * ky) % N];
-      // positions f and f + N/2 side by side: a thread's two columns (ky positions p and
-      // p + N/2, the same kz) read both factors in one 16-byte load
-      Fy[(size_t)j * N + (f % (N / 2)) * 2 + f / (N / 2)] =
-          make_float2((1.f - ry) * w0.x + ry * w1.x, (1.f - ry) * w0.y + ry * w1.y);
+      float* d = reinterpret_cast<float*>(Fy + ((size_t)j * NY + f % NY) * 2 + f / (2 * NY)) + f / NY % 2;
+      d[0] = (1.f - ry) * w0.x + ry * w1.x;
+      d[2] = (1.f - ry) * w0.y + ry * w1.y;
     } else {
       const int kz = f - N;
-      const int zi = s_yz[j].y;
+      const int zi = s_cell[j].z;
       const float rz = s_rr[j].y;
       const float2 w0 = tw[(zi * kz) % N], w1 = tw[((zi + 1) * kz) % N];
       Fz[(size_t)j * NZH + kz] = make_float2((1.f - rz) * w0.x + rz * w1.x, (1.f - rz) * w0.y + rz * w1.y);
     }
   }
+  // atoms per plane and per channel (ballots), then the lists: channels in order, planes ascending
+  // within a channel, atoms ascending within a plane
+  for (int x = warp; x < 8 * chunks + K; x += NW) {
+#pragma unroll
+    for (int wd = 0; wd < kDirectWords; ++wd) {
+      const int j = 32 * wd + lane;
+      const int4 c = j < na ? s_cell[j] : make_int4(-2, 0, 0, -2);
+      const int k = x - 8 * chunks;
+      const unsigned int m =
+          __ballot_sync(0xffffffffu, k < 0 ? (c.x == x || c.x + 1 == x) : j < na && (k == elec || c.w == k));
+      if (lane == 0) (k < 0 ? s_plane[x] : s_chan[k])[wd] = m;
+    }
+  }
   __syncthreads();
-  // per chunk, the atoms whose planes xi, xi + 1 meet it (warp 0, ballots in atom order)
-  const int jc0 = xlo >> 3, njc = (xhi >> 3) - jc0 + 1;  // planes < n: njc <= n / 8
-  if (tid < 32) {
-    for (int q = 0; q < njc; ++q) {
-      const int x0 = 8 * (jc0 + q);
-      for (int base = 0; base < 96; base += 32) {
-        const int j = base + tid;
-        const int o = j < na ? s_apk[j].x - x0 : -2;
-        const unsigned int m = __ballot_sync(0xffffffffu, o >= -1 && o <= 7);
-        if (tid == 0) s_cm[q][base >> 5] = m;
+  for (int i = tid; i < K * 8 * chunks; i += T) {
+    const int k = i / (8 * chunks), x = i - k * (8 * chunks);
+    uint32_t ch[kDirectWords];
+    int first = 0, total = 0;
+    for (int kk = 0; kk < k; ++kk)  // an atom has at most two entries per channel
+#pragma unroll
+      for (int wd = 0; wd < kDirectWords; ++wd) first += 2 * __popc(s_chan[kk][wd]);
+#pragma unroll
+    for (int wd = 0; wd < kDirectWords; ++wd) {
+      ch[wd] = s_chan[k][wd];
+      total += __popc(ch[wd]);
+    }
+    if (total) {
+      for (int y = 0; y < x; ++y)
+#pragma unroll
+        for (int wd = 0; wd < kDirectWords; ++wd) first += __popc(s_plane[y][wd] & ch[wd]);
+    }
+    int at = first;
+#pragma unroll
+    for (int wd = 0; wd < kDirectWords; ++wd)
+      for (unsigned int m = s_plane[x][wd] & ch[wd]; m; m &= m - 1) {
+        const int j = 32 * wd + __ffs(m) - 1;
+        const float4 w = s_w[j];
+        const bool own = s_cell[j].x == x;
+        const int wb = __float_as_int(k == elec ? (own ? w.z : w.w) : (own ? w.x : w.y));
+        s_list[at++] = make_int4(wb, wb, j * (NY * 2 * 16), j * (NZH * 8));
       }
-    }
+    s_run[k][x] = (uint32_t)first | (uint32_t)(at - first) << 16;
   }
   __syncthreads();
-  // Chunks of 8 planes: every thread owns columns, accumulates a chunk's planes in registers
-  // and visits the atoms touching the chunk in ascending order; an atom adds to planes xi and
-  // xi + 1, whose offsets in the chunk are the same for the whole CTA (a uniform switch).
-  // CPT columns per thread (c, c + NCOL / CPT, ...): the atom visit (list walk, weights, the
-  // offset switch) is shared by the columns, each column keeping its own accumulation order.
-  if (LOP && a.lop_tiled) {
-    for (int q = zlo; q <= zhi; ++q)
-      if (q < jc0 || q >= jc0 + njc)
-        for (int c = tid; c < NCOL; c += nthr) tiled_zero_chunk(a, r, k, q, c);
-  }
-  constexpr int CPT = kPlaneColsPerThread;
-  static_assert(NCOL % CPT == 0, "column split");
-  static_assert(CPT != 2 || (NCOL / 2) % NZH == 0, "paired columns share kz");
-  for (int cb = tid; cb < NCOL / CPT; cb += nthr) {
-    int kyp[CPT], kz[CPT];
-#pragma unroll
-    for (int u = 0; u < CPT; ++u) {
-      const int c = cb + u * (NCOL / CPT);
-      kyp[u] = c / NZH;
-      kz[u] = c - kyp[u] * NZH;
+  constexpr int BLOCKS = (Q + 31) / 32;
+  const int work = s_nitems * BLOCKS;
+  for (int b = blockIdx.x * NW + warp; b < work; b += gridDim.x * NW) {
+    const int it = s_item[b / BLOCKS], cb = (b % BLOCKS) * 32 + lane;
+    const int k = it & 15, q = (it >> 4) & 15;
+    if (cb >= Q) continue;
+    if (LOP && it >= 256) {
+      for (int i = 0; i < 4; ++i) tiled_zero_chunk(a, r, k, q, cb + i * Q);
+      continue;
     }
-    for (int q = 0; q < njc; ++q) {
-      const int jc = jc0 + q;
-      const int x0 = 8 * jc;
-      float ax[CPT][8], ay[CPT][8];
+    const int p = cb / NZH, kz = cb - p * NZH;
+    const unsigned char* fyb = reinterpret_cast<const unsigned char*>(Fy + p * 2);
+    const unsigned char* fzb = reinterpret_cast<const unsigned char*>(Fz + kz);
+    uint32_t hw[4][ROWS == kRowsBf16 ? 16 : 8];  // per column the rows' words (ROWS only)
+    pair_t px[2], py[2];                         // the even plane's sums
 #pragma unroll
-      for (int u = 0; u < CPT; ++u)
+    for (int d = 0; d < 8; ++d) {
+      pair_t ax[2] = {0ull, 0ull}, ay[2] = {0ull, 0ull};
+      const uint32_t run = s_run[k][8 * q + d];
+      const int4* e = s_list + (run & 0xffff);
+#pragma unroll 1
+      for (int cnt = run >> 16; cnt > 0; --cnt, ++e) {
+        const int4 en = *e;
+        const float4 f0 = *reinterpret_cast<const float4*>(fyb + en.z), f1 = *reinterpret_cast<const float4*>(fyb + en.z + 16);
+        const float2 fz = *reinterpret_cast<const float2*>(fzb + en.w);
+        const pair_t w = pk(__int_as_float(en.x), __int_as_float(en.y));
+        auto gx = [&](float x, float y) { return __fmaf_rn(x, fz.x, -__fmul_rn(y, fz.y)); };
+        auto gy = [&](float x, float y) { return __fmaf_rn(y, fz.x, __fmul_rn(x, fz.y)); };
+        ax[0] = p_fma(w, pk(gx(f0.x, f0.z), gx(f0.y, f0.w)), ax[0]);
+        ay[0] = p_fma(w, pk(gy(f0.x, f0.z), gy(f0.y, f0.w)), ay[0]);
+        ax[1] = p_fma(w, pk(gx(f1.x, f1.z), gx(f1.y, f1.w)), ax[1]);
+        ay[1] = p_fma(w, pk(gy(f1.x, f1.z), gy(f1.y, f1.w)), ay[1]);
+      }
+      if constexpr (!LOP) {
+        const int x = 8 * q + d;
+        if (x >= rec->xlo[k] && x <= rec->xhi[k]) {
+          float2* dst = a.A + (((size_t)r * K + k) * a.Lb + x) * NCOL + cb;
 #pragma unroll
-        for (int d = 0; d < 8; ++d) ax[u][d] = ay[u][d] = 0.f;
-      // only the atoms touching this chunk, in ascending order (the same for the whole CTA)
-      for (int wd = 0; wd < 3; ++wd) {
-        for (unsigned int mask = s_cm[q][wd]; mask; mask &= mask - 1) {
-          const int j = 32 * wd + __ffs(mask) - 1;
-          const int4 pk = s_apk[j];
-          const int o = pk.x - x0;
-          float gx[CPT], gy[CPT];
-          if constexpr (CPT == 2) {
-            // columns c and c + NCOL/2: ky positions p and p + N/2, one kz
-            const float4 fy2 = *reinterpret_cast<const float4*>(Fy + (size_t)j * N + 2 * kyp[0]);
-            const float2 fz = Fz[(size_t)j * NZH + kz[0]];
-            gx[0] = fy2.x * fz.x - fy2.y * fz.y;
-            gy[0] = fy2.x * fz.y + fy2.y * fz.x;
-            gx[1] = fy2.z * fz.x - fy2.w * fz.y;
-            gy[1] = fy2.z * fz.y + fy2.w * fz.x;
-          } else {
-#pragma unroll
-            for (int u = 0; u < CPT; ++u) {
-              const float2 fy = Fy[(size_t)j * N + (kyp[u] % (N / 2)) * 2 + kyp[u] / (N / 2)];
-              const float2 fz = Fz[(size_t)j * NZH + kz[u]];
-              gx[u] = fy.x * fz.x - fy.y * fz.y;
-              gy[u] = fy.x * fz.y + fy.y * fz.x;
-            }
+          for (int i = 0; i < 2; ++i) {
+            const float2 vx = unpk(ax[i]), vy = unpk(ay[i]);
+            dst[2 * i * Q] = make_float2(vx.x, vy.x);
+            dst[(2 * i + 1) * Q] = make_float2(vx.y, vy.y);
           }
-          const float w0 = __int_as_float(pk.y), w1 = __int_as_float(pk.z);
-          switch (o) {
-#define CDK_PLANE_PAIR(D)                                                  \
-  case D:                                                                  \
-    _Pragma("unroll") for (int u = 0; u < CPT; ++u) {                      \
-      ax[u][D] += w0 * gx[u];                                              \
-      ay[u][D] += w0 * gy[u];                                              \
-      ax[u][D + 1] += w1 * gx[u];                                          \
-      ay[u][D + 1] += w1 * gy[u];                                          \
-    }                                                                      \
-    break;
-            case -1:
+        }
+      } else if (d % 2 == 0) {
 #pragma unroll
-              for (int u = 0; u < CPT; ++u) {
-                ax[u][0] += w1 * gx[u];
-                ay[u][0] += w1 * gy[u];
-              }
-              break;
-            CDK_PLANE_PAIR(0)
-            CDK_PLANE_PAIR(1)
-            CDK_PLANE_PAIR(2)
-            CDK_PLANE_PAIR(3)
-            CDK_PLANE_PAIR(4)
-            CDK_PLANE_PAIR(5)
-            CDK_PLANE_PAIR(6)
-#undef CDK_PLANE_PAIR
-            default:  // o == 7: plane xi + 1 is the next chunk's
+        for (int i = 0; i < 2; ++i) {
+          px[i] = ax[i];
+          py[i] = ay[i];
+        }
+      } else {
+        // planes d - 1 and d (zero outside the channel's planes by construction) into the rows' words
 #pragma unroll
-              for (int u = 0; u < CPT; ++u) {
-                ax[u][7] += w0 * gx[u];
-                ay[u][7] += w0 * gy[u];
-              }
-              break;
+        for (int i = 0; i < 2; ++i) {
+          const float2 ex = unpk(px[i]), ey = unpk(py[i]), ox = unpk(ax[i]), oy = unpk(ay[i]);
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            uint32_t* w = hw[2 * i + u] + d / 2;
+            const float re0 = u ? ex.y : ex.x, re1 = u ? ox.y : ox.x, im0 = u ? ey.y : ey.x, im1 = u ? oy.y : oy.x;
+            if constexpr (ROWS == kRowsF16) {
+              const __half2 pr = __floats2half2_rn(re0, re1), pi = __floats2half2_rn(im0, im1);
+              w[0] = *reinterpret_cast<const uint32_t*>(&pr);
+              w[4] = *reinterpret_cast<const uint32_t*>(&pi);
+            } else {
+              split_bf16x2(re0, re1, w[0], w[8]);
+              split_bf16x2(im0, im1, w[4], w[12]);
+            }
           }
         }
       }
+    }
+    if constexpr (LOP) {
 #pragma unroll
-      for (int u = 0; u < CPT; ++u)
-        plane_chunk_write<N, LOP>(a, r, k, jc, x0, xlo, xhi, cb + u * (NCOL / CPT), ax[u], ay[u]);
+      for (int i = 0; i < 4; ++i) {
+        uint4 rows[ROWS == kRowsBf16 ? 4 : 2];
+#pragma unroll
+        for (int u = 0; u < (ROWS == kRowsBf16 ? 4 : 2); ++u)
+          rows[u] = make_uint4(hw[i][4 * u], hw[i][4 * u + 1], hw[i][4 * u + 2], hw[i][4 * u + 3]);
+        plane_rows_write<N, ROWS>(a, r, k, q, cb + i * Q, rows);
+      }
     }
   }
 }
@@ -1264,29 +1267,20 @@ constexpr size_t plane_smem() {
 }
 
 template <int N>
-size_t direct_smem(int cap) {
-  return sizeof(float2) * (N + (size_t)cap * (N + N / 2 + 1)) + sizeof(int4) * cap +
-         sizeof(int) * cap + (sizeof(int2) + sizeof(float2)) * cap;
-}
-
-template <int N>
 cudaError_t launch_spread_yz_t(const WaveArgs& a, cudaStream_t s) {
   const int cap = a.atom_cap > 0 ? a.atom_cap : a.max_atoms;
   if (a.kyof && cap <= kDirectMaxAtoms) {
-    const size_t sm = direct_smem<N>(cap);
-    if (a.lop) {
-      cudaError_t e = cudaFuncSetAttribute(k_spread_yz_direct<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    auto launch = [&](auto kern, size_t sm, int threads) {
+      const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
       if (e != cudaSuccess) return e;
-      WaveArgs b = a;
-      b.plane_rot_major = (a.lop_tiled && plane_rot_major_host()) ? 1 : 0;
-      const dim3 grid = b.plane_rot_major ? dim3(a.nrot, a.K) : dim3(a.K, a.nrot);
-      k_spread_yz_direct<N, true><<<grid, 256, sm, s>>>(b, a.kyof, cap);
+      // parts of a rotation's items: enough CTAs for small waves (each part repeats the tables)
+      const int parts = std::max(1, std::min(a.K, (148 * 6 + a.nrot - 1) / a.nrot));
+      kern<<<dim3(parts, a.nrot), threads, sm, s>>>(a, a.kyof, cap);
       return cudaGetLastError();
-    }
-    cudaError_t e = cudaFuncSetAttribute(k_spread_yz_direct<N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-    k_spread_yz_direct<N, false><<<dim3(a.K, a.nrot), 256, sm, s>>>(a, a.kyof, cap);
-    return cudaGetLastError();
+    };
+    if (!a.lop) return launch(k_spread_yz_direct<N, kRowsNone>, DirectShape<N, kRowsNone>::smem(cap), DirectShape<N, kRowsNone>::T);
+    if (a.f16) return launch(k_spread_yz_direct<N, kRowsF16>, DirectShape<N, kRowsF16>::smem(cap), DirectShape<N, kRowsF16>::T);
+    return launch(k_spread_yz_direct<N, kRowsBf16>, DirectShape<N, kRowsBf16>::smem(cap), DirectShape<N, kRowsBf16>::T);
   }
   if (a.lop) return cudaErrorInvalidValue;  // the FFT plane path writes A only
   const size_t sm = plane_smem<N>();

@@ -22,8 +22,7 @@
 //              idea; the coefficients come from traces of N^2 and N^3 and det N), and
 //              rmsd = sqrt(max(0, (Ga + Gb - 2 lambda) / n)). Cluster mode packs close(i, j) into
 //              one 32-bit word per warp with a ballot; matrix mode writes the RMSD itself.
-//   k_greedy   one CTA scans the candidates in order; thread t owns word t of the centre mask,
-//              so a candidate costs one row read and one __syncthreads_or.
+//   k_greedy   one CTA scans the candidates in order, 32 at a time.
 // All double arithmetic uses explicit round-to-nearest intrinsics (no contraction), sqrt and
 // division are IEEE, and every sum runs in atom order: the RMSDs are bit-identical to a host
 // double-precision evaluation of the same recipe without fused multiply-adds.
@@ -31,6 +30,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -50,28 +50,38 @@ __device__ __forceinline__ double dm(double a, double b) { return __dmul_rn(a, b
 __device__ __forceinline__ double da(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double ds(double a, double b) { return __dsub_rn(a, b); }
 
-// centred coordinates of conformer order[c] (or c) -> X[(a*3 + d) * ld + c], G[c]
-__global__ void k_center(int nConf, int nAtom, const double* __restrict__ coor,
-                         const int* __restrict__ sel, int nSel, const int* __restrict__ order,
-                         int ld, double* __restrict__ X, double* __restrict__ G) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nConf) return;
-  const double* p = coor + (size_t)(order ? order[c] : c) * nAtom * 3;
-  double s[3] = {0.0, 0.0, 0.0};
-  for (int i = 0; i < nSel; ++i)
-    for (int d = 0; d < 3; ++d) s[d] = da(s[d], p[sel[i] * 3 + d]);
-  double m[3];
-  for (int d = 0; d < 3; ++d) m[d] = __ddiv_rn(s[d], (double)nSel);
-  double g = 0.0;
-  for (int i = 0; i < nSel; ++i) {
-    double v[3];
-    for (int d = 0; d < 3; ++d) {
-      v[d] = ds(p[sel[i] * 3 + d], m[d]);
-      X[((size_t)i * 3 + d) * ld + c] = v[d];
-    }
-    g = da(g, da(da(dm(v[0], v[0]), dm(v[1], v[1])), dm(v[2], v[2])));
+// centred coordinates of conformer order[c] (or c) -> X[(a*3 + d) * ld + c], G[c]. CTA = 32
+// conformers: a thread per conformer and dimension for the mean and the centring, then one per
+// conformer for G. Bound by the latency of one conformer's sums, which run in atom order (bit-
+// identical to the host's): 23.7 us per 1,000 conformers of 40 atoms with one thread per conformer
+// and its dimensions one after the other, GPU time.
+constexpr int CL_CENTER = 32;
+__global__ void __launch_bounds__(3 * CL_CENTER) k_center(int nConf, int nAtom, const double* __restrict__ coor,
+                                                          const int* __restrict__ sel, int nSel,
+                                                          const int* __restrict__ order, int ld, double* X,
+                                                          double* __restrict__ G) {
+  const int c = blockIdx.x * CL_CENTER + threadIdx.x / 3, d = threadIdx.x % 3;
+  if (c < nConf) {
+    const double* p = coor + (size_t)(order ? order[c] : c) * nAtom * 3 + d;
+    double s = 0.0;
+#pragma unroll 8
+    for (int i = 0; i < nSel; ++i) s = da(s, p[sel[i] * 3]);
+    const double m = __ddiv_rn(s, (double)nSel);
+#pragma unroll 8
+    for (int i = 0; i < nSel; ++i) X[((size_t)i * 3 + d) * ld + c] = ds(p[sel[i] * 3], m);
   }
-  G[c] = g;
+  __syncthreads();
+  const int g = blockIdx.x * CL_CENTER + threadIdx.x;
+  if (threadIdx.x < CL_CENTER && g < nConf) {
+    double sum = 0.0;
+#pragma unroll 4
+    for (int i = 0; i < nSel; ++i) {
+      const double* v = X + (size_t)i * 3 * ld + g;
+      const double x = v[0], y = v[ld], z = v[2 * (size_t)ld];
+      sum = da(sum, da(da(dm(x, x), dm(y, y)), dm(z, z)));
+    }
+    G[g] = sum;
+  }
 }
 
 // minimum RMSD over rotations from the correlation S[p*3+q] = sum a_p b_q of centred sets
@@ -190,26 +200,62 @@ __global__ void __launch_bounds__(256) k_pairs(int nConf, int nSel, int ld,
   }
 }
 
-// the reference's greedy pass over candidates in energy order (positions), one CTA
+// The reference's greedy pass over candidates in energy order (positions), one CTA, 32 candidates
+// at a time: warp w tests candidate w of the block against the centres of the earlier blocks (all
+// lanes over the words of its row), then warp 0 settles the block in order, each candidate against
+// the block's own centres so far (one word). Two barriers per 32 candidates; one barrier per
+// candidate took 171 us for 1,000 conformers.
 __global__ void __launch_bounds__(1024) k_greedy(int nConf, int W, const uint32_t* __restrict__ bits,
                                                  const int* __restrict__ order, int maxCenters,
                                                  int* __restrict__ centers, int* __restrict__ count_out) {
-  const int t = threadIdx.x;
-  uint32_t cm = (t == 0) ? 1u : 0u;  // position 0 is the first centre
-  int count = 1;
-  if (t == 0) centers[0] = order[0];
-  for (int pi = 1; pi < nConf; ++pi) {
-    const int last = pi >> 5;
-    const uint32_t v = (t <= last && t < W) ? (bits[(size_t)pi * W + t] & cm) : 0u;
-    const int close = __syncthreads_or(v != 0u);
-    if (!close) {
-      if (t == last) cm |= 1u << (pi & 31);
-      if (t == 0) centers[count] = order[pi];
-      ++count;
+  __shared__ uint32_t s_cm[CL_MAX_CONF / 32];  // the centres so far, a bit per position
+  __shared__ uint32_t s_word[32];              // the candidates' words of their own block
+  __shared__ int s_close[32];
+  __shared__ int s_done;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (threadIdx.x == 0) s_done = 0;
+  int count = 0;  // warp 0's
+  for (int b = 0; b < W; ++b) {
+    const int pi = 32 * b + w;
+    const uint32_t* row = bits + (size_t)min(pi, nConf - 1) * W;
+    uint32_t v = 0;
+    for (int t = lane; t < b; t += 32) v |= row[t] & s_cm[t];
+    const bool close = __any_sync(0xffffffffu, v != 0);
+    if (lane == 0) {
+      s_close[w] = close;
+      s_word[w] = row[b];
     }
-    if (count == maxCenters) break;
+    __syncthreads();
+    if (w == 0) {
+      const uint32_t word = s_word[lane];
+      const unsigned int far = ~__ballot_sync(0xffffffffu, s_close[lane] != 0);
+      const int n = min(32, nConf - 32 * b);
+      uint32_t cmb = 0;
+      bool done = false;
+      for (int i = 0; i < n && !done; ++i) {
+        const uint32_t wi = __shfl_sync(0xffffffffu, word, i);
+        if (b == 0 && i == 0) {  // position 0 is the first centre, before any test of the count
+          cmb = 1u;
+          if (lane == 0) centers[0] = order[0];
+          count = 1;
+          continue;
+        }
+        if (((far >> i) & 1) && !(wi & cmb)) {
+          cmb |= 1u << i;
+          if (lane == 0) centers[count] = order[32 * b + i];
+          ++count;
+        }
+        done = count == maxCenters;
+      }
+      if (lane == 0) {
+        s_cm[b] = cmb;
+        s_done = done;
+      }
+    }
+    __syncthreads();
+    if (s_done) break;
   }
-  if (t == 0) *count_out = count;
+  if (threadIdx.x == 0) *count_out = count;
 }
 
 bool finite_all(const double* p, size_t n) {
@@ -226,23 +272,97 @@ std::vector<int> selected_atoms(int nAtom, const unsigned char* mask) {
   return sel;
 }
 
-struct ClusterBuffers {
-  double *coor = nullptr, *X = nullptr, *G = nullptr, *out = nullptr;
-  int *sel = nullptr, *order = nullptr, *centers = nullptr, *count = nullptr;
-  uint32_t* bits = nullptr;
+// Stream and device memory of a call. An allocation, its free and a stream cost 0.8 ms of a
+// 1,000-conformer call whose kernels take 0.12 ms (and an allocation up to 12 ms on a machine in use),
+// so a few are kept between calls: at most CL_IDLE of at most CL_KEEP bytes each, one call at a time
+// on each, given back to the device by cluster_release (cdk_ctx_destroy). The list itself is never
+// destroyed: no CUDA call runs while the process exits.
+constexpr size_t CL_KEEP = (size_t)32 << 20;
+constexpr size_t CL_IDLE = 2;
+struct ClusterSpace {
+  int dev = -1;
+  void* base = nullptr;
+  size_t cap = 0;
   cudaStream_t s = nullptr;
-  ~ClusterBuffers() {
-    if (s) cudaStreamSynchronize(s);
-    cudaFree(coor);
-    cudaFree(X);
-    cudaFree(G);
-    cudaFree(out);
-    cudaFree(sel);
-    cudaFree(order);
-    cudaFree(centers);
-    cudaFree(count);
-    cudaFree(bits);
+  void drop() {
+    int d = 0;
+    const bool moved = dev >= 0 && cudaGetDevice(&d) == cudaSuccess && d != dev;
+    if (moved) cudaSetDevice(dev);
+    if (base) cudaFree(base);
     if (s) cudaStreamDestroy(s);
+    if (moved) cudaSetDevice(d);
+    base = nullptr;
+    s = nullptr;
+    cap = 0;
+  }
+};
+struct ClusterIdle {
+  std::mutex mu;
+  std::vector<ClusterSpace> spaces;
+};
+ClusterIdle& cluster_idle() {
+  static ClusterIdle* const idle = new ClusterIdle;
+  return *idle;
+}
+
+// One call's buffers, carved from its space; every return waits for the stream and hands the space
+// back (or frees it: too large, or enough are kept)
+struct ClusterBuffers {
+  double *coor = nullptr, *X = nullptr, *G = nullptr;
+  int *sel = nullptr, *order = nullptr;
+  void* extra = nullptr;  // the caller's part
+  std::vector<int> idx;   // sel, then order: host source of an asynchronous copy
+  cudaStream_t s = nullptr;
+  ClusterSpace space;
+  cudaError_t take(size_t bytes) {
+    int d = 0;
+    cudaError_t e = cudaGetDevice(&d);
+    if (e != cudaSuccess) return e;
+    {
+      ClusterIdle& idle = cluster_idle();
+      std::lock_guard<std::mutex> lk(idle.mu);
+      for (size_t i = 0; i < idle.spaces.size() && space.dev < 0; ++i)
+        if (idle.spaces[i].dev == d) {
+          space = idle.spaces[i];
+          idle.spaces.erase(idle.spaces.begin() + i);
+        }
+    }
+    if (space.base) {
+      cudaPointerAttributes at{};
+      if (cudaPointerGetAttributes(&at, space.base) != cudaSuccess || at.type != cudaMemoryTypeDevice) {
+        (void)cudaGetLastError();
+        space = ClusterSpace{};  // the device was reset: memory and stream are gone
+      }
+    }
+    space.dev = d;
+    if (!space.s && (e = cudaStreamCreateWithFlags(&space.s, cudaStreamNonBlocking)) != cudaSuccess) {
+      space.s = nullptr;
+      return e;
+    }
+    s = space.s;
+    if (bytes > space.cap) {
+      if (space.base) cudaFree(space.base);
+      space.base = nullptr;
+      space.cap = 0;
+      if ((e = cudaMalloc(&space.base, bytes)) != cudaSuccess) {
+        space.base = nullptr;
+        return e;
+      }
+      space.cap = bytes;
+    }
+    return cudaSuccess;
+  }
+  ~ClusterBuffers() {
+    if (!space.s) return;
+    if (cudaStreamSynchronize(space.s) == cudaSuccess && space.base && space.cap <= CL_KEEP) {
+      ClusterIdle& idle = cluster_idle();
+      std::lock_guard<std::mutex> lk(idle.mu);
+      if (idle.spaces.size() < CL_IDLE) {
+        idle.spaces.push_back(space);
+        return;
+      }
+    }
+    space.drop();
   }
 };
 
@@ -255,25 +375,32 @@ struct ClusterBuffers {
     }                                                                     \
   } while (0)
 
-// shared set-up: copies, centring (in `order` when given); returns the leading dimension
+// shared set-up: memory (and `extra` bytes for the caller), copies, centring (in `order` when
+// given); returns the leading dimension
 int prepare(ClusterBuffers& b, int nConf, int nAtom, const double* coor,
-            const std::vector<int>& sel, const std::vector<int>* order, int* ld_out) {
+            const std::vector<int>& sel, const std::vector<int>* order, size_t extra, int* ld_out) {
+  auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
   const int ld = (nConf + CL_TGT - 1) / CL_TGT * CL_TGT;
   const int nSel = (int)sel.size();
-  CL_CUDA(cudaStreamCreateWithFlags(&b.s, cudaStreamNonBlocking));
-  CL_CUDA(cudaMalloc(&b.coor, sizeof(double) * (size_t)nConf * nAtom * 3));
-  CL_CUDA(cudaMalloc(&b.sel, sizeof(int) * nSel));
-  CL_CUDA(cudaMalloc(&b.X, sizeof(double) * (size_t)nSel * 3 * ld));
-  CL_CUDA(cudaMalloc(&b.G, sizeof(double) * ld));
+  const size_t b_coor = up(sizeof(double) * (size_t)nConf * nAtom * 3), b_X = up(sizeof(double) * (size_t)nSel * 3 * ld),
+               b_G = up(sizeof(double) * ld);
+  std::vector<int>& idx = b.idx;
+  idx = sel;
+  if (order) idx.insert(idx.end(), order->begin(), order->end());
+  const size_t b_idx = up(sizeof(int) * idx.size());
+  CL_CUDA(b.take(b_coor + b_X + b_G + b_idx + extra));
+  char* p = static_cast<char*>(b.space.base);
+  b.coor = reinterpret_cast<double*>(p);
+  b.X = reinterpret_cast<double*>(p + b_coor);
+  b.G = reinterpret_cast<double*>(p + b_coor + b_X);
+  b.sel = reinterpret_cast<int*>(p + b_coor + b_X + b_G);
+  b.order = order ? b.sel + nSel : nullptr;
+  b.extra = p + b_coor + b_X + b_G + b_idx;
   CL_CUDA(cudaMemcpyAsync(b.coor, coor, sizeof(double) * (size_t)nConf * nAtom * 3,
                           cudaMemcpyHostToDevice, b.s));
-  CL_CUDA(cudaMemcpyAsync(b.sel, sel.data(), sizeof(int) * nSel, cudaMemcpyHostToDevice, b.s));
-  if (order) {
-    CL_CUDA(cudaMalloc(&b.order, sizeof(int) * nConf));
-    CL_CUDA(cudaMemcpyAsync(b.order, order->data(), sizeof(int) * nConf, cudaMemcpyHostToDevice, b.s));
-  }
-  k_center<<<(nConf + 127) / 128, 128, 0, b.s>>>(nConf, nAtom, b.coor, b.sel, nSel, b.order, ld,
-                                                 b.X, b.G);
+  CL_CUDA(cudaMemcpyAsync(b.sel, idx.data(), sizeof(int) * idx.size(), cudaMemcpyHostToDevice, b.s));
+  k_center<<<(nConf + CL_CENTER - 1) / CL_CENTER, 3 * CL_CENTER, 0, b.s>>>(nConf, nAtom, b.coor, b.sel, nSel, b.order,
+                                                                           ld, b.X, b.G);
   CL_CUDA(cudaGetLastError());
   *ld_out = ld;
   return CDK_OK;
@@ -302,6 +429,14 @@ int check_inputs(int nConf, int nAtom, const double* coor, const unsigned char* 
 }
 
 }  // namespace
+
+void cluster_release() {
+  ClusterIdle& idle = cluster_idle();
+  std::lock_guard<std::mutex> lk(idle.mu);
+  for (ClusterSpace& sp : idle.spaces) sp.drop();
+  idle.spaces.clear();
+}
+
 }  // namespace cdk
 
 using namespace cdk;
@@ -328,26 +463,27 @@ extern "C" int cdk_cluster_conformers(int nConf, int nAtom, const double* coor,
   std::vector<int> order(idx.begin(), idx.end());
   ClusterBuffers b;
   int ld = 0;
-  rc = prepare(b, nConf, nAtom, coor, sel, &order, &ld);
-  if (rc != CDK_OK) return rc;
   const int W = (nConf + 31) / 32;
-  CL_CUDA(cudaMalloc(&b.bits, sizeof(uint32_t) * (size_t)nConf * W));
-  CL_CUDA(cudaMalloc(&b.centers, sizeof(int) * nConf));
-  CL_CUDA(cudaMalloc(&b.count, sizeof(int)));
+  // the result: the count, then the centres
+  const size_t b_bits = (sizeof(uint32_t) * (size_t)nConf * W + 255) & ~(size_t)255;
+  rc = prepare(b, nConf, nAtom, coor, sel, &order, b_bits + sizeof(int) * ((size_t)nConf + 1), &ld);
+  if (rc != CDK_OK) return rc;
+  uint32_t* bits = static_cast<uint32_t*>(b.extra);
+  int* result = reinterpret_cast<int*>(static_cast<char*>(b.extra) + b_bits);
   dim3 grid(W, (nConf + CL_REF - 1) / CL_REF);
-  k_pairs<<<grid, 256, 0, b.s>>>(nConf, (int)sel.size(), ld, b.X, b.G, cutoff, b.bits, W, nullptr);
+  k_pairs<<<grid, 256, 0, b.s>>>(nConf, (int)sel.size(), ld, b.X, b.G, cutoff, bits, W, nullptr);
   CL_CUDA(cudaGetLastError());
-  k_greedy<<<1, 1024, 0, b.s>>>(nConf, W, b.bits, b.order, maxCenters, b.centers, b.count);
+  k_greedy<<<1, 1024, 0, b.s>>>(nConf, W, bits, b.order, maxCenters, result + 1, result);
   CL_CUDA(cudaGetLastError());
-  int count = 0;
-  CL_CUDA(cudaMemcpyAsync(&count, b.count, sizeof(int), cudaMemcpyDeviceToHost, b.s));
+  std::vector<int> got((size_t)nConf + 1);
+  CL_CUDA(cudaMemcpyAsync(got.data(), result, sizeof(int) * got.size(), cudaMemcpyDeviceToHost, b.s));
   CL_CUDA(cudaStreamSynchronize(b.s));
+  const int count = got[0];
   if (count < 1 || count > nConf) {
     set_error("clustering returned an invalid centre count");
     return CDK_ERR_CUDA;
   }
-  CL_CUDA(cudaMemcpyAsync(centers, b.centers, sizeof(int) * count, cudaMemcpyDeviceToHost, b.s));
-  CL_CUDA(cudaStreamSynchronize(b.s));
+  std::copy(got.begin() + 1, got.begin() + 1 + count, centers);
   *nCenters = count;
   return CDK_OK;
 }
@@ -363,13 +499,13 @@ extern "C" int cdk_pair_rmsd(int nConf, int nAtom, const double* coor,
   }
   ClusterBuffers b;
   int ld = 0;
-  rc = prepare(b, nConf, nAtom, coor, sel, nullptr, &ld);
+  rc = prepare(b, nConf, nAtom, coor, sel, nullptr, sizeof(double) * (size_t)nConf * nConf, &ld);
   if (rc != CDK_OK) return rc;
-  CL_CUDA(cudaMalloc(&b.out, sizeof(double) * (size_t)nConf * nConf));
+  double* d_out = static_cast<double*>(b.extra);
   dim3 grid((nConf + CL_TGT - 1) / CL_TGT, (nConf + CL_REF - 1) / CL_REF);
-  k_pairs<<<grid, 256, 0, b.s>>>(nConf, (int)sel.size(), ld, b.X, b.G, 0.0, nullptr, 0, b.out);
+  k_pairs<<<grid, 256, 0, b.s>>>(nConf, (int)sel.size(), ld, b.X, b.G, 0.0, nullptr, 0, d_out);
   CL_CUDA(cudaGetLastError());
-  CL_CUDA(cudaMemcpyAsync(out, b.out, sizeof(double) * (size_t)nConf * nConf, cudaMemcpyDeviceToHost, b.s));
+  CL_CUDA(cudaMemcpyAsync(out, d_out, sizeof(double) * (size_t)nConf * nConf, cudaMemcpyDeviceToHost, b.s));
   CL_CUDA(cudaStreamSynchronize(b.s));
   return CDK_OK;
 }

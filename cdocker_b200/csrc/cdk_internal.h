@@ -188,6 +188,8 @@ cudaError_t launch_group_rotations(const RotDesc* rots, const ConfDesc* confs, c
                                    const AtomParam* params, long nrot, int max_atoms, int K, float h,
                                    int jc, void* scratch, RotDesc** sorted, cudaStream_t s);
 cudaError_t launch_spread_yz(const WaveArgs& a, cudaStream_t s);
+// FP32 planes into a.A, then split-BF16 ligand rows of them into a.lop (both layouts)
+cudaError_t launch_rows_from_planes(const WaveArgs& a, cudaStream_t s);
 cudaError_t launch_xpass(const WaveArgs& a, cudaStream_t s);
 cudaError_t launch_yz_inv_argmin(const WaveArgs& a, cudaStream_t s);
 // the inverse (y,z) pass over paired planes (WaveArgs.bpairs), and the key pairs per rotation it
@@ -239,8 +241,10 @@ int stream_bgroup();
 cudaError_t launch_top_build(int n, int K, const float2* pt, void* top, const float* f16_scale,
                              cudaStream_t s);
 cudaError_t launch_xpass_stream(const WaveArgs& a, const void* top, cudaStream_t s);
-// true when launch_spread_yz takes the direct plane path (the only one that can write lop)
+// true when launch_spread_yz takes the direct plane path (the only one that can write lop); with
+// split-BF16 rows it takes larger ligands
 bool direct_planes(const WaveArgs& a);
+bool direct_rows_bf16(const WaveArgs& a);
 
 // tcgen05 x pass with the Hankel operator resident in shared memory (any n, ligand box <= 32
 // planes): its shape for (n, K, box, form) and its launch (k_tile_plan, then the x pass)

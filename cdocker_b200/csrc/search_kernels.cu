@@ -244,6 +244,12 @@ __device__ __forceinline__ void plane_forward(float2* P, float2* O, int npairs,
 }
 
 // ---------------------------------------------------------------------------------------
+// an atom on the plane being spread: y and z cells and ratios, its weight times the x weight
+struct SpreadAtom {
+  double yr, zr, w;
+  int yi, zi;
+};
+
 // spread + forward (y,z) transform of one (rotation, channel, x plane)
 template <int N>
 __global__ void __launch_bounds__(256) k_spread_yz(WaveArgs a) {
@@ -264,57 +270,73 @@ __global__ void __launch_bounds__(256) k_spread_yz(WaveArgs a) {
   float* Pf = reinterpret_cast<float*>(P);
   for (int i = tid; i < npairs * (N + 1); i += nthr) P[i] = make_float2(0.f, 0.f);
   __syncthreads();
-  // spread the atoms touching plane x (src/FillLigandGrid.cpp:24-66 vdW, :75-118 elec).
-  // Warp 0 adds the atoms one after another in ascending atom order, the four (y,z) corners
-  // of an atom in four lanes (they never share a cell), each add rounded back to float from
-  // double as in the reference: the plane is bit-identical to FillLigandGrid's and the
-  // search is deterministic whatever the batch around a rotation.
-  const RotDesc rd = a.rots[r];
-  const ConfDesc cd = a.confs[rd.conf];
-  const AtomParam* prm = a.params + cd.param_off;
+  // spread the atoms touching plane x (src/FillLigandGrid.cpp:24-66 vdW, :75-118 elec). The cells
+  // and ratios of up to 256 atoms at a time by a thread each, compacted in ascending order; then
+  // warp 0 adds the atoms one after another, the four (y,z) corners of an atom in four lanes (they
+  // never share a cell), the weights of eight atoms computed together, each add rounded back to
+  // float from double as in the reference: the plane is bit-identical to FillLigandGrid's and the
+  // search is deterministic whatever the batch around a rotation. (With the divisions of an atom's
+  // cells and ratios in warp 0's loop as well, 2.14 against 1.98 ms per 1,000 rotations of a 100-atom
+  // ligand at 64^3.)
+  __shared__ int s_warp[8];
+  __shared__ SpreadAtom s_at[256];
+  const AtomParam* prm = a.params + rec->param_off;
   const float mn0 = rec->mn[0], mn1 = rec->mn[1], mn2 = rec->mn[2];
   const float h = a.spacing;
   const bool elec = (k == a.K - 1);
   const int nA = rec->nA;
-  if (tid < 32) {
-    const int lane = tid;
-    for (int base = 0; base < nA; base += 32) {
-      const int i = base + lane;
-      bool touch = false;
-      if (i < nA) {
-        const AtomParam ap = prm[i];
-        if (elec || ap.slot == k) {
-          const int xi = cell_of(a.rot_xyz[(size_t)r * a.max_atoms + i].x, mn0, h);
-          touch = (xi == x) || (xi + 1 == x);
-        }
-      }
-      unsigned int m = __ballot_sync(0xffffffffu, touch);
-      while (m) {
-        const int at = base + __ffs(m) - 1;
-        m &= m - 1;
-        if (lane < 4) {
-          const AtomParam ap = prm[at];
-          const float4 p = a.rot_xyz[(size_t)r * a.max_atoms + at];
-          const int xi = cell_of(p.x, mn0, h);
-          const double xr = ratio_of(p.x, mn0, h, xi);
-          const double wx = (xi == x) ? __dsub_rn(1.0, xr) : xr;
-          const int yi = cell_of(p.y, mn1, h), zi = cell_of(p.z, mn2, h);
-          const double yr = ratio_of(p.y, mn1, h, yi), zr = ratio_of(p.z, mn2, h, zi);
-          const double sc = elec ? (double)ap.charge : (double)ap.w_vdw;
-          const int dy = lane >> 1, dz = lane & 1;
-          const double w = __dmul_rn(__dmul_rn(__dmul_rn(sc, wx), dy ? yr : __dsub_rn(1.0, yr)),
-                                     dz ? zr : __dsub_rn(1.0, zr));
-          const int y = yi + dy, z = zi + dz;
-          if (y < N && z < N) {
-            float* cell = &Pf[((y >> 1) * (N + 1) + z) * 2 + (y & 1)];
-            *cell = (float)__dadd_rn((double)*cell, w);
-          }
-        }
-        __syncwarp();
+  for (int base = 0; base < nA; base += 256) {
+    const int i = base + tid, lane = tid & 31;
+    bool touch = false;
+    int xi = 0;
+    float4 p;
+    AtomParam ap;
+    if (i < nA) {
+      ap = prm[i];
+      if (elec || ap.slot == k) {
+        p = a.rot_xyz[(size_t)r * a.max_atoms + i];
+        xi = cell_of(p.x, mn0, h);
+        touch = (xi == x) || (xi + 1 == x);
       }
     }
+    const unsigned int m = __ballot_sync(0xffffffffu, touch);
+    if (lane == 0) s_warp[tid >> 5] = __popc(m);
+    __syncthreads();
+    int at = 0, cnt = 0;
+    for (int w = 0; w < 8; ++w) {
+      if (w < (tid >> 5)) at += s_warp[w];
+      cnt += s_warp[w];
+    }
+    if (touch) {
+      const double xr = ratio_of(p.x, mn0, h, xi);
+      SpreadAtom sa;
+      sa.yi = cell_of(p.y, mn1, h);
+      sa.zi = cell_of(p.z, mn2, h);
+      sa.yr = ratio_of(p.y, mn1, h, sa.yi);
+      sa.zr = ratio_of(p.z, mn2, h, sa.zi);
+      sa.w = __dmul_rn(elec ? (double)ap.charge : (double)ap.w_vdw, (xi == x) ? __dsub_rn(1.0, xr) : xr);
+      s_at[at + __popc(m & ((1u << lane) - 1))] = sa;
+    }
+    __syncthreads();
+    if (tid < 32) {
+      for (int j0 = 0; j0 < cnt; j0 += 8) {
+        const int j = j0 + (lane >> 2), dy = (lane >> 1) & 1, dz = lane & 1;
+        float* cell = nullptr;
+        double w = 0.0;
+        if (j < cnt) {
+          const SpreadAtom sa = s_at[j];
+          w = __dmul_rn(__dmul_rn(sa.w, dy ? sa.yr : __dsub_rn(1.0, sa.yr)), dz ? sa.zr : __dsub_rn(1.0, sa.zr));
+          const int y = sa.yi + dy, z = sa.zi + dz;
+          if (y < N && z < N) cell = &Pf[((y >> 1) * (N + 1) + z) * 2 + (y & 1)];
+        }
+        for (int o = 0; o < min(8, cnt - j0); ++o) {
+          if ((lane >> 2) == o && cell) *cell = (float)__dadd_rn((double)*cell, w);
+          __syncwarp();
+        }
+      }
+    }
+    __syncthreads();
   }
-  __syncthreads();
   plane_forward<N>(P, O, npairs, tw);
   // write the plane's half spectrum (16-byte stores)
   float4* dst = reinterpret_cast<float4*>(a.A + (((size_t)r * a.K + k) * a.Lb + x) * NCOL);
@@ -382,8 +404,51 @@ __device__ __forceinline__ void tile_plan_range(const WaveArgs& a, int r, int k,
     }
 }
 
-constexpr int kDirectMaxAtoms = 96;
-constexpr int kDirectWords = kDirectMaxAtoms / 32;
+// Split-BF16 ligand rows from FP32 planes (A), for ligands that the direct plane kernel does not
+// take: per (rotation, channel) the chunks of the tile's stage plan (tiled rows; zeros where the
+// channel has no plane) or its own chunks. Bound: DRAM (8 bytes read and, with the hi and lo parts,
+// 8 written per plane and column); two columns per thread, so that loads and stores are 16 and 128
+// bytes.
+template <int N>
+__global__ void __launch_bounds__(256) k_rows_from_planes(const __grid_constant__ WaveArgs a) {
+  constexpr int NCOL = N * (N / 2 + 1);
+  const int r = blockIdx.x, k = blockIdx.y;
+  const RotRec* rec = a.rec + r;
+  if (!rec->valid) return;
+  const int xlo = rec->xlo[k], xhi = rec->xhi[k];
+  int lo = 1, hi = 0;
+  if (xlo <= xhi) lo = xlo >> 3, hi = xhi >> 3;
+  if (a.lop_tiled) tile_plan_range(a, r, k, lo, hi);
+  const float2* src = a.A + ((size_t)r * a.K + k) * a.Lb * NCOL;
+  for (int i = threadIdx.x; i < (hi - lo + 1) * (NCOL / 2); i += 256) {
+    const int q = lo + i / (NCOL / 2), c = i % (NCOL / 2) * 2;
+    uint32_t h[2][16];
+#pragma unroll
+    for (int d = 0; d < 8; d += 2) {
+      float4 v[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int x = 8 * q + d + e;
+        v[e] = x >= xlo && x <= xhi ? *reinterpret_cast<const float4*>(src + (size_t)x * NCOL + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+      split_bf16x2(v[0].x, v[1].x, h[0][d / 2], h[0][8 + d / 2]);
+      split_bf16x2(v[0].y, v[1].y, h[0][4 + d / 2], h[0][12 + d / 2]);
+      split_bf16x2(v[0].z, v[1].z, h[1][d / 2], h[1][8 + d / 2]);
+      split_bf16x2(v[0].w, v[1].w, h[1][4 + d / 2], h[1][12 + d / 2]);
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      uint4 rows[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) rows[j] = make_uint4(h[u][4 * j], h[u][4 * j + 1], h[u][4 * j + 2], h[u][4 * j + 3]);
+      plane_rows_write<N, kRowsBf16>(a, r, k, q, c + u, rows);
+    }
+  }
+}
+
+// Largest ligand of the direct plane kernel: 96 atoms; split-BF16 rows up to 128 (FP32 planes stay
+// with FillLigandGrid's rounding above 96, and the split-FP16 form refuses larger ligands)
+constexpr int direct_max_atoms(int rows) { return rows == kRowsBf16 ? 128 : 96; }
 
 // Shape of the direct plane kernel: threads per CTA and CTAs per SM asked for (registers), shared
 // memory for ligands of at most cap atoms
@@ -431,6 +496,7 @@ __global__ void __launch_bounds__(DirectShape<N, ROWS>::T, DirectShape<N, ROWS>:
   float2* Fz = reinterpret_cast<float2*>(Fy + (size_t)cap * NY * 2);  // [cap][NZH]
   float2* tw = Fz + (size_t)cap * NZH;                             // [N]
   float2* s_rr = tw + N;                                           // [cap] y and z ratios
+  constexpr int kDirectWords = direct_max_atoms(ROWS) / 32;
   __shared__ uint32_t s_plane[N][kDirectWords];   // atoms with a cell on the plane (bit j)
   __shared__ uint32_t s_chan[KMAX][kDirectWords];  // atoms of the channel
   __shared__ uint32_t s_run[KMAX][N];             // list entries of (channel, plane): first | count << 16
@@ -1269,7 +1335,7 @@ constexpr size_t plane_smem() {
 template <int N>
 cudaError_t launch_spread_yz_t(const WaveArgs& a, cudaStream_t s) {
   const int cap = a.atom_cap > 0 ? a.atom_cap : a.max_atoms;
-  if (a.kyof && cap <= kDirectMaxAtoms) {
+  if (a.kyof && cap <= direct_max_atoms(!a.lop ? kRowsNone : a.f16 ? kRowsF16 : kRowsBf16)) {
     auto launch = [&](auto kern, size_t sm, int threads) {
       const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
       if (e != cudaSuccess) return e;
@@ -1509,15 +1575,34 @@ cudaError_t launch_prep(const WaveArgs& a, cudaStream_t s) {
 cudaError_t launch_spread_yz(const WaveArgs& a, cudaStream_t s) {
   if (a.lop_tiled) {
     // the tiled rows zero-fill by the tiles' stage plans: k_tile_plan first
-    if (!a.lop || !direct_planes(a) || (reinterpret_cast<uintptr_t>(a.lop) & 127)) return cudaErrorInvalidValue;
+    if (!a.lop || !(a.f16 ? direct_planes(a) : direct_rows_bf16(a)) || (reinterpret_cast<uintptr_t>(a.lop) & 127)) return cudaErrorInvalidValue;
     cudaError_t e = launch_tile_plan(a, (a.Lb + 7) / 8, s);
     if (e != cudaSuccess) return e;
   }
   CDK_DISPATCH_N(a.n, launch_spread_yz_t, a, s);
 }
+template <int N>
+static cudaError_t launch_rows_t(const WaveArgs& a, cudaStream_t s) {
+  k_rows_from_planes<N><<<dim3(a.nrot, a.K), 256, 0, s>>>(a);
+  return cudaGetLastError();
+}
+cudaError_t launch_rows_from_planes(const WaveArgs& a, cudaStream_t s) {
+  if (!a.A || !a.lop || a.f16 || (reinterpret_cast<uintptr_t>(a.lop) & 127)) return cudaErrorInvalidValue;
+  WaveArgs p = a;  // the planes first, then the rows
+  p.lop = nullptr;
+  p.lop_tiled = 0;
+  cudaError_t e = launch_spread_yz(p, s);
+  if (e == cudaSuccess && a.lop_tiled) e = launch_tile_plan(a, (a.Lb + 7) / 8, s);
+  if (e != cudaSuccess) return e;
+  CDK_DISPATCH_N(a.n, launch_rows_t, a, s);
+}
 bool direct_planes(const WaveArgs& a) {
   const int cap = a.atom_cap > 0 ? a.atom_cap : a.max_atoms;
-  return a.kyof != nullptr && cap <= kDirectMaxAtoms;
+  return a.kyof != nullptr && cap <= direct_max_atoms(kRowsNone);
+}
+bool direct_rows_bf16(const WaveArgs& a) {
+  const int cap = a.atom_cap > 0 ? a.atom_cap : a.max_atoms;
+  return a.kyof != nullptr && cap <= direct_max_atoms(kRowsBf16);
 }
 cudaError_t launch_yz_inv_argmin(const WaveArgs& a, cudaStream_t s) {
   if (a.bpairs) return launch_yz_pairs(a, s);

@@ -16,14 +16,15 @@
 // pipe 51 %, per thread and channel about 430 instructions of which 226 floating point and 42 shared
 // loads). Measured on a B200, K = 9, against the radix kernel that exchanged between the stages for
 // every channel (its issue slots went to shared-memory traffic and block barriers): 32^3, 500
-// rotations 0.373 -> 0.159 ms; 64^3, 5,000 rotations 15.1 -> 7.5 ms; 96^3, 999 rotations 10.7 -> 4.1
+// rotations 0.373 -> 0.145 ms; 64^3, 5,000 rotations 15.1 -> 7.2 ms; 96^3, 999 rotations 10.7 -> 4.2
 // ms; 128^3, 1,000 rotations 26.1 -> 11.1 ms; results bit-identical.
 //
 // CTA = 8 columns x a chunk of rotations; its 8-column tile of the receptor spectra stays in
 // shared memory. 8 columns and not 16 or 32: the tile fits beside the rings at every n and K <=
 // 16, a spectra load is shared by the warp's four rotations, and 64-byte row pieces still fill
-// whole sectors. G groups of 128 threads (G = 4 at n <= 64, 3 above: the registers of the
-// second stage) each take every G-th set of 4 rotations; a warp's lanes are 8 columns x 4
+// whole sectors. G groups of 128 threads (7 at n = 32, 4 at 64, 3 above: the registers of the second
+// stage; at 32^3 seven measured 0.145 ms against 0.162 with four, 500 rotations, and 0.99 against 1.12,
+// 4,000; at 64^3 five, at 96 registers, gained nothing) each take every G-th set of 4 rotations; a warp's lanes are 8 columns x 4
 // rotations. A set's channels are streamed through a ring of nst stages by 16-byte cp.async (one
 // stage: the planes 0 .. R1 JN - 1 of one channel, the untouched ones zero-filled by the copy),
 // one 128-thread barrier per channel.
@@ -52,7 +53,7 @@ constexpr size_t kXpSmemCap = 227 * 1024 - 512;
 template <int N>
 struct XpShape {
   static constexpr int R1 = N / 8;
-  static constexpr int GMAX = N <= 64 ? 4 : 3;  // groups of 128 threads
+  static constexpr int GMAX = N == 32 ? 7 : N == 64 ? 4 : 3;  // groups of 128 threads
 };
 
 // twiddles w_N^(np q) of the output pairs (q, q + 4), q = 0..3, in the kernel's parameters: real,
@@ -503,7 +504,7 @@ bool xp_plan(const WaveArgs& a, XpPlan* p) {
   const int R1 = a.n / 8, ncol = a.n * (a.n / 2 + 1);
   const int jn = (a.Lb + R1 - 1) / R1;
   p->jm = jn <= 2 ? 2 : jn <= 4 ? jn : 8;
-  p->G = a.n <= 64 ? XpShape<64>::GMAX : XpShape<128>::GMAX;
+  p->G = a.n == 32 ? XpShape<32>::GMAX : a.n == 64 ? XpShape<64>::GMAX : XpShape<128>::GMAX;
   p->nst = 3;
   int most = XP_MAX_CHUNK;
   while (xp_layout(a.n, a.K, p->G, p->nst, R1 * p->jm, most).total > kXpSmemCap) {

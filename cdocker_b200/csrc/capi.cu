@@ -490,12 +490,12 @@ int run_waves(cdk_ctx* c, const float* d_coor, const AtomParam* d_params, const 
     if (prof) CDK_CUDA(cudaEventRecordWithFlags(ev[3], s, evflags));
     CDK_CUDA(launch_yz_inv_argmin(a, s));
     if (tiebreak) CDK_CUDA(launch_tiebreak(a, c->d_grids, f16form ? 1e-3f : 1e-4f, s));
-    if (topk > 0)
-      CDK_CUDA(launch_topk_rescore(a, c->d_grids, topk, static_cast<TopPose*>(c->topk.base) + (size_t)waves * topk, s));
     if (prof) CDK_CUDA(cudaEventRecordWithFlags(ev[4], s, evflags));
-    CDK_CUDA(launch_finalize(a, s));
+    if (topk > 0)
+      CDK_CUDA(launch_finalize_topk(a, c->d_grids, topk, static_cast<TopPose*>(c->topk.base) + (size_t)waves * topk, s));
+    else CDK_CUDA(launch_finalize(a, s));
     if (prof) CDK_CUDA(cudaEventRecordWithFlags(ev[5], s, evflags));
-    launches += kLaunchesPerWave + (rows ? 1 : convert ? 2 : 0) + (tiebreak ? 1 : 0) + (topk > 0 ? 1 : 0);  // + k_tile_plan (and the rows of planes)
+    launches += kLaunchesPerWave + (rows ? 1 : convert ? 2 : 0) + (tiebreak ? 1 : 0);  // + k_tile_plan (and the rows of planes)
     ++waves;
   }
   c->kev_used = prof ? (int)waves : 0;

@@ -177,7 +177,8 @@ struct TopPose {
   int pad;
   double e64;  // its FP64 direct grid-energy sum
 };
-cudaError_t launch_topk_rescore(const WaveArgs& a, const float* grids, int k, TopPose* out, cudaStream_t s);
+// launch_finalize, and the k lowest poses of the wave with their FP64 re-score into top[0 .. k)
+cudaError_t launch_finalize_topk(const WaveArgs& a, const float* grids, int k, TopPose* top, cudaStream_t s);
 // FP64 near-tie break of the argmin over the planes' two smallest keys (a.keys2), before
 // launch_finalize; grids: the receptor grids [K][n][n][n]
 cudaError_t launch_tiebreak(const WaveArgs& a, const float* grids, float tol, cudaStream_t s);

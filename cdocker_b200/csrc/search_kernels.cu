@@ -1077,48 +1077,67 @@ __global__ void __launch_bounds__(32 * kOctWarps, 3) k_yz_octet(WaveArgs a) {
   }
 }
 
-// FP64 energy of rotation r at translation (ti, tj, tk): the direct trilinear grid-energy sum
-// over its rotated atoms (k_prep's rot_xyz and min corner), cells and ratios in
-// FillLigandGrid's arithmetic, accumulated in double across the warp's lanes (atoms).
-__device__ double pose_energy_fp64(const WaveArgs& a, const float* grids, int r, int ti, int tj, int tk,
-                                   int lane) {
+// FP64 energies of rotation r at P translations (linear indices lin[]): the direct trilinear
+// grid-energy sum over its rotated atoms (k_prep's rot_xyz and min corner), cells and ratios in
+// FillLigandGrid's arithmetic, accumulated in double across the warp's lanes (atoms). A few rotations
+// per warp at most, so it is a chain of memory latencies: an atom's 16 P grid values are loaded
+// before the first is used, and a tie's two translations go together (64^3, 61 rotations: tie break 15 ->
+// 12 us with the caches cold).
+template <int P>
+__device__ void pose_energies_fp64(const WaveArgs& a, const float* grids, int r, const unsigned int* lin,
+                                   int lane, double* e) {
   const RotRec* rec = a.rec + r;
-  const RotDesc rd = a.rots[r];
-  const ConfDesc cd = a.confs[rd.conf];
-  const AtomParam* prm = a.params + cd.param_off;
+  const AtomParam* prm = a.params + rec->param_off;
   const int n = a.n, K = a.K;
   const size_t Ng = (size_t)n * n * n;
   const float h = a.spacing;
-  double e = 0.0;
+#pragma unroll
+  for (int q = 0; q < P; ++q) e[q] = 0.0;
   for (int i = lane; i < rec->nA; i += 32) {
     const float4 p4 = a.rot_xyz[(size_t)r * a.max_atoms + i];
+    const AtomParam ap = prm[i];
     const float p[3] = {p4.x, p4.y, p4.z};
+    const bool vdw = ap.slot >= 0 && ap.slot < K - 1;
     int ci[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) ci[d] = cell_of(p[d], rec->mn[d], h);
+    float gv[P][8], ge[P][8];
+    bool in[P][8];
+#pragma unroll
+    for (int q = 0; q < P; ++q) {
+      const int x = ci[0] + (int)(lin[q] / (n * n)), y = ci[1] + (int)((lin[q] / n) % n), z = ci[2] + (int)(lin[q] % n);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const int gx = x + ((c >> 2) & 1), gy = y + ((c >> 1) & 1), gz = z + (c & 1);
+        in[q][c] = gx < n && gy < n && gz < n;
+        const size_t g = ((size_t)gx * n + gy) * n + gz;
+        gv[q][c] = in[q][c] && vdw ? grids[(size_t)ap.slot * Ng + g] : 0.f;
+        ge[q][c] = in[q][c] ? grids[(size_t)(K - 1) * Ng + g] : 0.f;
+      }
+    }
     double rr[3];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      ci[d] = cell_of(p[d], rec->mn[d], h);
-      rr[d] = ratio_of(p[d], rec->mn[d], h, ci[d]);
-    }
-    const AtomParam ap = prm[i];
+    for (int d = 0; d < 3; ++d) rr[d] = ratio_of(p[d], rec->mn[d], h, ci[d]);
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
       const int dx = (c >> 2) & 1, dy = (c >> 1) & 1, dz = c & 1;
-      const int gx = ci[0] + dx + ti, gy = ci[1] + dy + tj, gz = ci[2] + dz + tk;
-      if (gx >= n || gy >= n || gz >= n) continue;
       const double w = (dx ? rr[0] : 1.0 - rr[0]) * (dy ? rr[1] : 1.0 - rr[1]) * (dz ? rr[2] : 1.0 - rr[2]);
-      const size_t g = ((size_t)gx * n + gy) * n + gz;
-      if (ap.slot >= 0 && ap.slot < K - 1) e += (double)ap.w_vdw * w * (double)grids[(size_t)ap.slot * Ng + g];
-      e += (double)ap.charge * w * (double)grids[(size_t)(K - 1) * Ng + g];
+#pragma unroll
+      for (int q = 0; q < P; ++q) {
+        if (!in[q][c]) continue;
+        if (vdw) e[q] += (double)ap.w_vdw * w * (double)gv[q][c];
+        e[q] += (double)ap.charge * w * (double)ge[q][c];
+      }
     }
   }
-  for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
-  return e;
+#pragma unroll
+  for (int q = 0; q < P; ++q)
+    for (int o = 16; o > 0; o >>= 1) e[q] += __shfl_xor_sync(0xffffffffu, e[q], o);
 }
 
 // FP64 near-tie break of the argmin (precision forms), warp per rotation: the two smallest keys
 // over the rotation's key pairs (one per window plane, or WaveArgs.key_slots); when the second energy lies within tol * max(|E1|, 1) of
-// the first, both translations are re-scored in FP64 (pose_energy_fp64) and the lower one is
+// the first, both translations are re-scored in FP64 (pose_energies_fp64) and the lower one is
 // kept -- the smaller linear index (x-major first) on an exact FP64 tie. The reported energy
 // stays the search's own value at the kept translation. work[4] counts re-scored rotations,
 // work[5] the ones whose translation changed.
@@ -1142,8 +1161,10 @@ __global__ void __launch_bounds__(128) k_tiebreak(WaveArgs a, const float* __res
   const float e1 = key_to_float((unsigned int)(b1 >> 32)), e2 = key_to_float((unsigned int)(b2 >> 32));
   if (!(e2 - e1 <= tol * fmaxf(fabsf(e1), 1.f))) return;
   const unsigned int l1 = (unsigned int)b1, l2 = (unsigned int)b2;
-  const double f1 = pose_energy_fp64(a, grids, r, l1 / (n * n), (l1 / n) % n, l1 % n, lane);
-  const double f2 = pose_energy_fp64(a, grids, r, l2 / (n * n), (l2 / n) % n, l2 % n, lane);
+  const unsigned int lin[2] = {l1, l2};
+  double f[2];
+  pose_energies_fp64<2>(a, grids, r, lin, lane, f);
+  const double f1 = f[0], f2 = f[1];
   if (lane == 0) {
     const bool flip = f2 < f1 || (f2 == f1 && l2 < l1);
     if (flip) a.keys[r] = b2;
@@ -1154,35 +1175,46 @@ __global__ void __launch_bounds__(128) k_tiebreak(WaveArgs a, const float* __res
   }
 }
 
-// FP64 re-score of the k lowest-energy poses of a wave (precision forms), one CTA: the k
+// FP64 re-score of the k lowest-energy poses of a wave (precision forms), one CTA of k_finalize: the k
 // smallest final keys (energy, then the rotation's place in the wave) by k rounds of a block
 // minimum over each thread's own sorted candidates, then one warp per pose for its FP64 direct
 // grid-energy sum at its kept translation. out[j]: the rotation's output slot, the search's
 // energy, its translation's linear index and the FP64 energy; unused slots get out = -1.
-__global__ void __launch_bounds__(256) k_topk_rescore(WaveArgs a, const float* __restrict__ grids, int k,
-                                                      TopPose* __restrict__ out) {
+// L: the candidates a thread keeps (k of them are enough). The loads of four rotations are issued
+// together: the other blocks are done long before this one.
+template <int L>
+__device__ void topk_rescore(const WaveArgs& a, const float* __restrict__ grids, int k,
+                             TopPose* __restrict__ out) {
   __shared__ unsigned long long s_min[8];
-  __shared__ unsigned long long s_pick[kTopMax];
+  __shared__ unsigned long long s_pick[L];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // per thread: its kTopMax smallest (energy bits, rotation) keys, ascending
-  unsigned long long cand[kTopMax];
+  // per thread: its L smallest (energy bits, rotation) keys, ascending
+  unsigned long long cand[L];
 #pragma unroll
-  for (int j = 0; j < kTopMax; ++j) cand[j] = ~0ull;
-  for (int r = tid; r < a.nrot; r += blockDim.x) {
-    const RotRec* rec = a.rec + r;
-    const unsigned long long key = a.keys[r];
-    if (!rec->valid || key == ~0ull) continue;
-    unsigned long long c = (key & 0xffffffff00000000ull) | (unsigned int)r;
+  for (int j = 0; j < L; ++j) cand[j] = ~0ull;
+  for (int r0 = tid; r0 < a.nrot; r0 += 4 * blockDim.x) {
+    unsigned long long key[4];
 #pragma unroll
-    for (int j = 0; j < kTopMax; ++j) {
-      const unsigned long long lo = c < cand[j] ? c : cand[j];
-      c = c < cand[j] ? cand[j] : c;
-      cand[j] = lo;
+    for (int u = 0; u < 4; ++u) {
+      const int r = r0 + u * (int)blockDim.x;
+      key[u] = r < a.nrot && a.rec[r].valid ? a.keys[r] : ~0ull;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (key[u] == ~0ull) continue;
+      unsigned long long c = (key[u] & 0xffffffff00000000ull) | (unsigned int)(r0 + u * (int)blockDim.x);
+      if (c >= cand[L - 1]) continue;
+#pragma unroll
+      for (int j = 0; j < L; ++j) {
+        const unsigned long long lo = c < cand[j] ? c : cand[j];
+        c = c < cand[j] ? cand[j] : c;
+        cand[j] = lo;
+      }
     }
   }
   int head = 0;
   for (int j = 0; j < k; ++j) {
-    unsigned long long m = head < kTopMax ? cand[0] : ~0ull;
+    unsigned long long m = head < L ? cand[0] : ~0ull;
     for (int o = 16; o > 0; o >>= 1) {
       const unsigned long long v = __shfl_xor_sync(0xffffffffu, m, o);
       m = v < m ? v : m;
@@ -1195,8 +1227,8 @@ __global__ void __launch_bounds__(256) k_topk_rescore(WaveArgs a, const float* _
     // the owner pops its head (keys are unique: one rotation each)
     if (g != ~0ull && cand[0] == g) {
 #pragma unroll
-      for (int q = 0; q + 1 < kTopMax; ++q) cand[q] = cand[q + 1];
-      cand[kTopMax - 1] = ~0ull;
+      for (int q = 0; q + 1 < L; ++q) cand[q] = cand[q + 1];
+      cand[L - 1] = ~0ull;
       ++head;
     }
     __syncthreads();
@@ -1211,8 +1243,8 @@ __global__ void __launch_bounds__(256) k_topk_rescore(WaveArgs a, const float* _
     if (g != ~0ull) {
       const int r = (int)(unsigned int)g;
       const unsigned int lin = (unsigned int)a.keys[r];
-      const int n = a.n;
-      const double e64 = pose_energy_fp64(a, grids, r, lin / (n * n), (lin / n) % n, lin % n, lane);
+      double e64;
+      pose_energies_fp64<1>(a, grids, r, &lin, lane, &e64);
       tp.out = a.rots[r].out;
       tp.lin = (int)lin;
       tp.e = key_to_float((unsigned int)(a.keys[r] >> 32));
@@ -1222,8 +1254,18 @@ __global__ void __launch_bounds__(256) k_topk_rescore(WaveArgs a, const float* _
   }
 }
 
-__global__ void k_finalize(WaveArgs a) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+// Results of the final keys. TOP: block 0 re-scores the k lowest-energy poses (it reads the same keys, so
+// beside the other blocks and not in a launch before them: 64^3, 61 rotations, 14.5 us and a launch of
+// 8 -> 14 together; the whole search 298 -> 278)
+template <bool TOP>
+__global__ void __launch_bounds__(256) k_finalize(WaveArgs a, const float* __restrict__ grids, int k,
+                                                  TopPose* __restrict__ top) {
+  if (TOP && blockIdx.x == 0) {
+    if (k <= 8) topk_rescore<8>(a, grids, k, top);
+    else topk_rescore<kTopMax>(a, grids, k, top);
+    return;
+  }
+  const int r = (blockIdx.x - (TOP ? 1 : 0)) * blockDim.x + threadIdx.x;
   if (r >= a.nrot) return;
   const int out = a.rots[r].out;
   const RotRec* rec = a.rec + r;
@@ -1608,18 +1650,18 @@ cudaError_t launch_yz_inv_argmin(const WaveArgs& a, cudaStream_t s) {
   if (a.bpairs) return launch_yz_pairs(a, s);
   CDK_DISPATCH_N(a.n, launch_yz_inv_t, a, s);
 }
-cudaError_t launch_topk_rescore(const WaveArgs& a, const float* grids, int k, TopPose* out, cudaStream_t s) {
-  if (!grids || !out || k < 1 || k > kTopMax) return cudaErrorInvalidValue;
-  k_topk_rescore<<<1, 256, 0, s>>>(a, grids, k, out);
-  return cudaGetLastError();
-}
 cudaError_t launch_tiebreak(const WaveArgs& a, const float* grids, float tol, cudaStream_t s) {
   if (!a.keys2 || !grids) return cudaErrorInvalidValue;
   k_tiebreak<<<(a.nrot + 3) / 4, 128, 0, s>>>(a, grids, tol);
   return cudaGetLastError();
 }
 cudaError_t launch_finalize(const WaveArgs& a, cudaStream_t s) {
-  k_finalize<<<(a.nrot + 255) / 256, 256, 0, s>>>(a);
+  k_finalize<false><<<(a.nrot + 255) / 256, 256, 0, s>>>(a, nullptr, 0, nullptr);
+  return cudaGetLastError();
+}
+cudaError_t launch_finalize_topk(const WaveArgs& a, const float* grids, int k, TopPose* top, cudaStream_t s) {
+  if (!grids || !top || k < 1 || k > kTopMax) return cudaErrorInvalidValue;
+  k_finalize<true><<<(a.nrot + 255) / 256 + 1, 256, 0, s>>>(a, grids, k, top);
   return cudaGetLastError();
 }
 cudaError_t launch_finalize_server(const WaveArgs& a, float* ebase, int* ibase, cudaStream_t s) {

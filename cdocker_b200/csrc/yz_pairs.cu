@@ -9,7 +9,8 @@
 // bytes), either as plane pairs (FP32 x pass) or as plane quads (one-column Hankel x pass, whose
 // stores must fill 32-byte sectors).
 //
-// CTA = a rotation and a part of its plane pairs, looped. An octet of 8 lanes owns a line (a kz
+// k_yz_pairs (k_yz_quads, for plane quads at n <= 64, is described there): CTA = a rotation and a part of
+// its plane pairs, looped. An octet of 8 lanes owns a line (a kz
 // column for y, a row pair for z): lane t takes block t in the first stage and the groups np = t,
 // t + 8, ... in the second; the exchange between them goes through the line's own storage in the
 // plane buffer, with __syncwarp only, so that a pair of planes has two CTA barriers (y -> z, z -> the
@@ -70,6 +71,90 @@ __device__ __forceinline__ float min_nan(float a, float b) {
   float r;
   asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
   return r;
+}
+
+// Energies of z = np + R1 j, j < 8, of rows y (real parts) and y + 1 (imaginary parts) and planes x, x + 1,
+// into the thread's smallest key (TOP2: two smallest). Called by whole warps; on: the lane has values.
+// s_bound: order_key of an energy that at least one (TOP2: two) of the CTA's values so far does not
+// exceed: a value strictly above it cannot enter.
+template <int N, bool TOP2>
+__device__ __forceinline__ void yz_keep(const cpair* u, bool on, int np, int x, int y, bool row1, bool plane1, int Wz,
+                                        float inv, int lane, unsigned int* s_bound, unsigned long long& best,
+                                        unsigned long long& best2) {
+  constexpr int R1 = N / 8;
+  float lo = INFINITY;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    if (on && np + R1 * j < Wz) {
+      const float2 e0 = unpk(u[j].x), e1 = unpk(u[j].y);
+      float m = row1 ? min_nan(e0.x, e1.x) : e0.x;
+      if (plane1) m = min_nan(m, row1 ? min_nan(e0.y, e1.y) : e0.y);
+      lo = min_nan(lo, m);
+    }
+  }
+  lo *= inv;
+  const unsigned int seen = *(volatile unsigned int*)s_bound;
+  float bound = key_to_float(seen);
+  if (__any_sync(0xffffffffu, on && !(lo > bound))) {
+    // the bound that this warp's lines give: two (TOP2) lanes hold an energy no larger
+    const unsigned int k = on ? order_key(lo) : 0xffffffffu;
+    unsigned int m = __reduce_min_sync(0xffffffffu, k);
+    if (TOP2 && __popc(__ballot_sync(0xffffffffu, k == m)) < 2)
+      m = __reduce_min_sync(0xffffffffu, k == m ? 0xffffffffu : k);
+    if (m < seen) {
+      bound = key_to_float(m);
+      if (lane == 0) atomicMin(s_bound, m);
+    }
+    if (on && !(lo > bound)) {
+      const unsigned int lin = (unsigned int)((x * N + y) * N + np);
+      auto keep = [&](float e, unsigned int at) {
+        e *= inv;
+        if (e > bound) return;
+        const unsigned long long key = ((unsigned long long)order_key(e) << 32) | at;
+        if constexpr (TOP2) top2_insert(key, best, best2);
+        else best = key < best ? key : best;
+      };
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (np + R1 * j < Wz) {
+          const float2 e0 = unpk(u[j].x), e1 = unpk(u[j].y);
+          const unsigned int at = lin + (unsigned int)(R1 * j);
+          keep(e0.x, at);
+          if (row1) keep(e1.x, at + N);
+          if (plane1) {
+            keep(e0.y, at + N * N);
+            if (row1) keep(e1.y, at + N * N + N);
+          }
+        }
+      }
+    }
+  }
+}
+
+// The CTA's smallest keys, reduced in the plane buffer (free by now) and stored
+template <int N, int NW, bool TOP2>
+__device__ __forceinline__ void yz_store(const WaveArgs& a, int r, int part, void* buffer, unsigned long long best,
+                                         unsigned long long best2) {
+  const int tid = threadIdx.x;
+  warp_keep_min<TOP2>(best, best2);
+  unsigned long long* s_best = static_cast<unsigned long long*>(buffer);
+  if ((tid & 31) == 0) {
+    s_best[tid >> 5] = best;
+    if constexpr (TOP2) s_best[NW + (tid >> 5)] = best2;
+  }
+  __syncthreads();
+  if (tid < 32) {
+    best = tid < NW ? s_best[tid] : ~0ull;
+    if constexpr (TOP2) best2 = tid < NW ? s_best[NW + tid] : ~0ull;
+    warp_keep_min<TOP2>(best, best2);
+    if (tid == 0) {
+      atomicMin(a.keys + r, best);
+      if constexpr (TOP2) {
+        a.keys2[((size_t)r * N + part) * 2] = best;
+        a.keys2[((size_t)r * N + part) * 2 + 1] = best2;
+      }
+    }
+  }
 }
 
 template <int N, bool TOP2, bool QUADS>
@@ -180,78 +265,190 @@ __global__ void __launch_bounds__(YzShape<N>::T, YzShape<N>::CTAS) k_yz_pairs(co
         for (int b = 0; b < 8; ++b) u[b] = ld(A + b * R1 + ((on ? np : 0) ^ (R1 % 8 == 0 ? b : b >> 1)));
         yz_twiddle<N>(u, tw, on ? np : 0);
         PairRadix<8, +1>::run(u);
-        // energies of z = np + R1 j: rows y (real parts) and y + 1 (imaginary parts), planes x, x + 1
-        float lo = INFINITY;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          if (on && np + R1 * j < Wz) {
-            const float2 e0 = unpk(u[j].x), e1 = unpk(u[j].y);
-            float m = row1 ? min_nan(e0.x, e1.x) : e0.x;
-            if (plane1) m = min_nan(m, row1 ? min_nan(e0.y, e1.y) : e0.y);
-            lo = min_nan(lo, m);
-          }
-        }
-        lo *= inv;
-        const unsigned int seen = *(volatile unsigned int*)&s_bound;
-        float bound = key_to_float(seen);
-        if (__any_sync(0xffffffffu, on && !(lo > bound))) {
-          // the bound that this warp's lines give: two (TOP2) lanes hold an energy no larger
-          const unsigned int k = on ? order_key(lo) : 0xffffffffu;
-          unsigned int m = __reduce_min_sync(0xffffffffu, k);
-          if (TOP2 && __popc(__ballot_sync(0xffffffffu, k == m)) < 2)
-            m = __reduce_min_sync(0xffffffffu, k == m ? 0xffffffffu : k);
-          if (m < seen) {
-            bound = key_to_float(m);
-            if (lane == 0) atomicMin(&s_bound, m);
-          }
-          if (on && !(lo > bound)) {
-            const unsigned int lin = (unsigned int)((x * N + y) * N + np);
-            auto keep = [&](float e, unsigned int at) {
-              e *= inv;
-              if (e > bound) return;
-              const unsigned long long key = ((unsigned long long)order_key(e) << 32) | at;
-              if constexpr (TOP2) top2_insert(key, best, best2);
-              else best = key < best ? key : best;
-            };
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              if (np + R1 * j < Wz) {
-                const float2 e0 = unpk(u[j].x), e1 = unpk(u[j].y);
-                const unsigned int at = lin + (unsigned int)(R1 * j);
-                keep(e0.x, at);
-                if (row1) keep(e1.x, at + N);
-                if (plane1) {
-                  keep(e0.y, at + N * N);
-                  if (row1) keep(e1.y, at + N * N + N);
-                }
-              }
-            }
-          }
-        }
+        yz_keep<N, TOP2>(u, on, np, x, y, row1, plane1, Wz, inv, lane, &s_bound, best, best2);
       }
     }
     __syncthreads();
   }
-  // the CTA's smallest keys; the plane buffer is free
-  warp_keep_min<TOP2>(best, best2);
-  unsigned long long* s_best = reinterpret_cast<unsigned long long*>(O);
-  constexpr int NW = T / 32;
-  if ((tid & 31) == 0) {
-    s_best[tid >> 5] = best;
-    if constexpr (TOP2) s_best[NW + (tid >> 5)] = best2;
+  yz_store<N, T / 32, TOP2>(a, r, part, O, best, best2);
+}
+
+// Plane quads of single rotations (n <= 64: the one-column Hankel x pass): a CTA loads a quad's four
+// planes, contiguous in B, into its plane buffer with one bulk copy per row, so no load goes through the
+// LSU -- there a 16-byte load, whose lanes took half of 32 sectors in 8 or more lines, cost 24 L1 cycles,
+// 42 % of the L1 time at 64^3 -- and transforms both pairs in place between the same two barriers. Three
+// CTAs per SM at 64^3 hide each other's copies. Units of 16 bytes (one pair of one column) lie column by
+// column, pair by pair; a quarter-warp is 2 columns x 2 pairs x 2 blocks in y and 4 positions x 2 pairs in
+// z, 8 different banks with rows and blocks 4 mod 8 units apart. ms per 1e5 rotations (two smallest
+// keys): 64^3 33.3 -> 28.8, 32^3 5.6 -> 4.4 against k_yz_pairs over the same quads; over plane pairs (FP32 x
+// pass, two shorter copies per row) the same scheme lost, 30.6 against 28.0 at 64^3.
+template <int N>
+struct YzQuadShape {
+  static constexpr int NZH = N / 2 + 1;
+  static constexpr int T = N == 32 ? 160 : 288;
+  static constexpr int CTAS = N == 32 ? 6 : 3;
+  static constexpr int UNITS = 2 * NZH;  // of a row
+  static constexpr int ROW = (UNITS + 3) / 8 * 8 + 4;
+  static constexpr int BLOCK = (N / 8) * ROW + 4;
+  static constexpr size_t SMEM = sizeof(float4) * ((N / 8) * 7 + 8 * BLOCK);
+  static_assert(ROW >= UNITS && ROW % 8 == 4 && BLOCK % 8 == 4, "row and block strides");
+  static_assert(ROW + UNITS >= 2 * N, "a row pair holds a line of both pairs");
+};
+
+constexpr long kYzWaitLimit = 1l << 22;
+
+template <int N, bool TOP2>
+__global__ void __launch_bounds__(YzQuadShape<N>::T, YzQuadShape<N>::CTAS) k_yz_quads(const __grid_constant__ WaveArgs a) {
+  using S = YzQuadShape<N>;
+  constexpr int NZH = S::NZH, R1 = N / 8, T = S::T, NW = T / 32, ROW = S::ROW, BLOCK = S::BLOCK;
+  static_assert(R1 <= 8 && b_quad_rots(N) == 1, "one second-stage group per lane, rotations apart");
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float4* tw = reinterpret_cast<float4*>(smem_raw);
+  float4* O = tw + R1 * 7;
+  __shared__ unsigned int s_bound;
+  __shared__ __align__(8) uint64_t s_full;
+  __shared__ int s_fail;
+  const int r = blockIdx.y, part = blockIdx.x, parts = gridDim.x;
+  const RotRec* rec = a.rec + r;
+  if (!rec->valid) return;
+  const int Wx = rec->W[0], Wy = rec->W[1], Wz = rec->W[2];
+  const int quads = (Wx + 3) / 4, npairs = (Wy + 1) / 2;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t full = (uint32_t)__cvta_generic_to_shared(&s_full);
+  for (int i = tid; i < R1 * 7; i += T) {
+    const float2 w = a.tw[(i / 7) * (i % 7 + 1)];
+    tw[i] = make_float4(w.x, w.x, w.y, w.y);
   }
-  __syncthreads();
-  if (tid < 32) {
-    best = tid < NW ? s_best[tid] : ~0ull;
-    if constexpr (TOP2) best2 = tid < NW ? s_best[NW + tid] : ~0ull;
-    warp_keep_min<TOP2>(best, best2);
-    if (tid == 0) {
-      atomicMin(a.keys + r, best);
-      if constexpr (TOP2) {
-        a.keys2[((size_t)r * N + part) * 2] = best;
-        a.keys2[((size_t)r * N + part) * 2 + 1] = best2;
+  if (tid == 0) {
+    s_bound = order_key(INFINITY);
+    s_fail = 0;
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  auto ld = [](const float4* p) {
+    const float4 f = *p;
+    return cpair{pk(f.x, f.y), pk(f.z, f.w)};
+  };
+  auto st = [](float4* p, cpair v) {
+    const float2 x = unpk(v.x), y = unpk(v.y);
+    *p = make_float4(x.x, x.y, y.x, y.y);
+  };
+  // warp 0: the quad's rows into the plane buffer (row f = block f / R1, position f % R1)
+  auto load_quad = [&](int p) {
+    constexpr uint32_t bytes = NZH * 32;
+    if (lane == 0)
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%1], %0;" ::"r"(bytes * N), "r"(full) : "memory");
+    __syncwarp();
+    const float4* src = reinterpret_cast<const float4*>(a.B) + b_quad_index<N>(r, 0) + (size_t)p * (N * NZH * 2);
+    for (int f = lane; f < N; f += 32)
+      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                       (uint32_t)__cvta_generic_to_shared(O + (f / R1) * BLOCK + (f % R1) * ROW)),
+                   "l"(src + (size_t)f * (NZH * 2)), "r"(bytes), "r"(full)
+                   : "memory");
+  };
+  auto wait_quad = [&](uint32_t parity) {
+    for (long i = 0; i < kYzWaitLimit; ++i) {
+      uint32_t done;
+      asm volatile(
+          "{\n\t.reg .pred p;\n\t"
+          "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+          "selp.u32 %0, 1, 0, p;\n\t}"
+          : "=r"(done)
+          : "r"(full), "r"(parity)
+          : "memory");
+      if (done) return;
+      if (i > 32) {
+        if (*(volatile int*)&s_fail) return;  // another thread gave up
+        __nanosleep(40);
       }
     }
+    *(volatile int*)&s_fail = 1;
+  };
+  const int q = lane & 1;                          // the lane's pair of the quad
+  const int ty = lane >> 2;                        // y: block or group; columns 2u, 2u + 1 of unit u
+  const int t = (lane >> 1) & 7, g2 = lane >> 4;   // z: place in the line; row pairs 2w, 2w + 1 of unit w
+  constexpr int SW = R1 - 1;  // swizzle of a line's positions b R1 + m -> b R1 + (m ^ (b & SW))
+  const float inv = 1.0f / (float)((double)N * N * N);
+  unsigned long long best = ~0ull, best2 = ~0ull;
+  __syncthreads();
+  if (warp == 0 && part < quads) load_quad(part);
+  uint32_t parity = 0;
+#pragma unroll 1
+  for (int p = part; p < quads; p += parts, parity ^= 1u) {
+    wait_quad(parity);
+    // y: both stages of columns 2u, 2u + 1 and both pairs by one warp
+#pragma unroll 1
+    for (int u = warp; u < (NZH + 1) / 2; u += NW) {
+      const int c = 2 * u + ((lane >> 1) & 1);
+      const bool has_col = c < NZH;
+      float4* const col = O + (has_col ? 2 * c + q : 0);
+      if (has_col) {
+        cpair v[R1];
+#pragma unroll
+        for (int j = 0; j < R1; ++j) v[j] = ld(col + ty * BLOCK + j * ROW);
+        PairRadix<R1, +1>::run(v);
+#pragma unroll
+        for (int j = 0; j < R1; ++j) st(col + ty * BLOCK + j * ROW, v[j]);
+      }
+      __syncwarp();
+      if (has_col && ty < R1) {
+        cpair v[8];
+#pragma unroll
+        for (int b = 0; b < 8; ++b) v[b] = ld(col + b * BLOCK + ty * ROW);
+        yz_twiddle<N>(v, tw, ty);
+        PairRadix<8, +1>::run(v);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) st(col + j * BLOCK + ty * ROW, v[j]);
+      }
+    }
+    __syncthreads();
+    // z: rows (2g, 2g + 1) as one complex line with its Hermitian extension
+    const int x = 4 * p + 2 * q;
+    const bool pair = x < Wx, plane1 = x + 1 < Wx;
+#pragma unroll 1
+    for (int w = warp; 2 * w < npairs; w += NW) {
+      const int g = 2 * w + g2;
+      const bool act = g < npairs && pair;
+      const int y = 2 * (g < npairs ? g : 0);
+      float4* const A = O + (y / R1) * BLOCK + (y % R1) * ROW + q;
+      const float4* const Bv = A + ROW;
+      {
+        cpair z[R1];
+#pragma unroll
+        for (int j = 0; j < R1; ++j) {
+          const int k = t + 8 * j;
+          const int m = j < R1 / 2 ? k : N - k;
+          const cpair ak = ld(A + 2 * m), bk = ld(Bv + 2 * m);
+          if (j < R1 / 2) z[j] = cpair{p_sub(ak.x, bk.y), p_add(ak.y, bk.x)};
+          else z[j] = cpair{p_add(ak.x, bk.y), p_sub(bk.x, ak.y)};
+          if ((j == 0 || j == R1 / 2) && t == 0) z[j] = cpair{ak.x, bk.x};  // k = 0, N / 2
+        }
+        __syncwarp();  // the warp has read its rows: their slots become the exchange
+        PairRadix<R1, +1>::run(z);
+        if (g < npairs) {
+#pragma unroll
+          for (int j = 0; j < R1; ++j) st(A + 2 * (t * R1 + (j ^ (t & SW))), z[j]);
+        }
+        __syncwarp();
+      }
+      const bool on = act && t < R1;
+      cpair v[8];
+#pragma unroll
+      for (int b = 0; b < 8; ++b) v[b] = ld(A + 2 * (b * R1 + ((t & SW) ^ (b & SW))));
+      yz_twiddle<N>(v, tw, t & SW);
+      PairRadix<8, +1>::run(v);
+      yz_keep<N, TOP2>(v, on, t & SW, x, y, y + 1 < Wy, plane1, Wz, inv, lane, &s_bound, best, best2);
+    }
+    // the next quad's copies (async proxy) follow every read and write of this one
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    if (warp == 0 && p + parts < quads) load_quad(p + parts);
+  }
+  yz_store<N, NW, TOP2>(a, r, part, O, best, best2);
+  if (tid == 0 && s_fail) {
+    atomicOr(a.fault, 1);
+    s_fail = 0;
+    wait_quad(parity ^ 1u);  // a copy still in flight lands before the CTA leaves
   }
 }
 
@@ -263,14 +460,26 @@ int yz_parts(int nrot) {
   return (int)std::max<long>(1, std::min<long>(N / 4, (want + nrot - 1) / nrot));
 }
 
+// Over quads of single rotations (n <= 64) k_yz_quads, else k_yz_pairs: both sides above
 template <int N>
 cudaError_t launch_t(const WaveArgs& a, cudaStream_t s) {
-  const bool quads = a.bpairs == 4;
-  auto kern = a.keys2 ? (quads ? k_yz_pairs<N, true, true> : k_yz_pairs<N, true, false>)
-                      : (quads ? k_yz_pairs<N, false, true> : k_yz_pairs<N, false, false>);
-  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)YzShape<N>::SMEM);
+  constexpr bool SINGLE = b_quad_rots(N) == 1;
+  if (a.bpairs == 2 && a.keys2) return cudaErrorInvalidValue;  // plane pairs are the FP32 form's: one key
+  void (*kern)(WaveArgs) = k_yz_pairs<N, false, false>;
+  size_t sm = YzShape<N>::SMEM;
+  int threads = YzShape<N>::T;
+  if (a.bpairs == 4) {
+    if constexpr (SINGLE) {
+      kern = a.keys2 ? k_yz_quads<N, true> : k_yz_quads<N, false>;
+      sm = YzQuadShape<N>::SMEM;
+      threads = YzQuadShape<N>::T;
+    } else {
+      kern = a.keys2 ? k_yz_pairs<N, true, true> : k_yz_pairs<N, false, true>;
+    }
+  }
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
-  kern<<<dim3(yz_parts<N>(a.nrot), a.nrot), YzShape<N>::T, YzShape<N>::SMEM, s>>>(a);
+  kern<<<dim3(yz_parts<N>(a.nrot), a.nrot), threads, sm, s>>>(a);
   return cudaGetLastError();
 }
 

@@ -49,20 +49,22 @@ struct YzShape {
   // units of 16 bytes between rows, and between blocks of R1 rows: both 4 mod 8
   static constexpr int ROW = (NZH + 3) / 8 * 8 + 4;
   static constexpr int BLOCK = (N / 8) * ROW + 4;
-  static constexpr size_t SMEM = sizeof(float4) * ((N / 8) * 7 + 8 * BLOCK);
+  static constexpr size_t SMEM = sizeof(float2) * (N / 8) * 7 + sizeof(float4) * 8 * BLOCK;
   static_assert(ROW >= NZH && ROW % 8 == 4 && BLOCK % 8 == 4, "row and block strides");
 };
 
-// Twiddle products v[k] conj(w^(np k)), k = 1..7, of both planes; table [np][k - 1] of (c, c, s, s)
+// Twiddle products v[k] conj(w^(np k)), k = 1..7, of both planes; table [np][k - 1] of (c, s): loads of 8
+// bytes and not the doubled pairs (c, c, s, s) cost half the wavefronts (inverse pass 96^3 FP32 1.31 ->
+// 1.25 ms, 128^3 3.38 -> 3.21)
 template <int N>
-__device__ __forceinline__ void yz_twiddle(cpair* v, const float4* tw, int np) {
+__device__ __forceinline__ void yz_twiddle(cpair* v, const float2* tw, int np) {
 #pragma unroll
   for (int k = 1; k < 8; ++k) {
-    const float4 w = tw[np * 7 + k - 1];
-    const pair_t c = pk(w.x, w.y), s = pk(w.z, w.w);
+    const float2 w = tw[np * 7 + k - 1];
+    const pair_t c = pk(w.x, w.x), s = pk(w.y, w.y);
     const float2 y = unpk(v[k].y), t = unpk(p_mul(v[k].x, s));
     v[k].x = p_fma(v[k].x, c, p_mul(v[k].y, s));
-    v[k].y = pk(__fmaf_rn(y.x, w.x, -t.x), __fmaf_rn(y.y, w.y, -t.y));
+    v[k].y = pk(__fmaf_rn(y.x, w.x, -t.x), __fmaf_rn(y.y, w.x, -t.y));
   }
 }
 
@@ -162,10 +164,10 @@ __global__ void __launch_bounds__(YzShape<N>::T, YzShape<N>::CTAS) k_yz_pairs(co
   constexpr int NZH = N / 2 + 1, NCOL = N * NZH, R1 = N / 8, T = YzShape<N>::T;
   constexpr int ROW = YzShape<N>::ROW, BLOCK = YzShape<N>::BLOCK;
   constexpr int NG = (R1 + 7) / 8;  // second-stage groups per lane
-  static_assert(T / 8 >= N / 2, "an octet per row pair");
+  static_assert(T / 8 >= N / 2 && R1 * 7 % 2 == 0, "an octet per row pair; the plane buffer aligned");
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float4* tw = reinterpret_cast<float4*>(smem_raw);
-  float4* O = tw + R1 * 7;
+  float2* tw = reinterpret_cast<float2*>(smem_raw);
+  float4* O = reinterpret_cast<float4*>(tw + R1 * 7);
   // order_key of an energy that at least one (TOP2: two) of the CTA's values so far does not exceed:
   // a value strictly above it cannot enter
   __shared__ unsigned int s_bound;
@@ -178,10 +180,7 @@ __global__ void __launch_bounds__(YzShape<N>::T, YzShape<N>::CTAS) k_yz_pairs(co
   // y: octets of lanes 4 apart, so that a quarter-warp holds 4 neighbouring columns of 2 blocks
   const int ty = lane >> 2, gy = (tid >> 5) * 4 + (lane & 3);
   const int t = tid & 7, g = tid >> 3;  // z: octets of consecutive lanes
-  for (int i = tid; i < R1 * 7; i += T) {
-    const float2 w = a.tw[(i / 7) * (i % 7 + 1)];
-    tw[i] = make_float4(w.x, w.x, w.y, w.y);
-  }
+  for (int i = tid; i < R1 * 7; i += T) tw[i] = a.tw[(i / 7) * (i % 7 + 1)];
   if (tid == 0) s_bound = order_key(INFINITY);
   auto ld = [](const float4* p) {
     const float4 f = *p;
@@ -274,12 +273,13 @@ __global__ void __launch_bounds__(YzShape<N>::T, YzShape<N>::CTAS) k_yz_pairs(co
 }
 
 // Plane quads of single rotations (n <= 64: the one-column Hankel x pass): a CTA loads a quad's four
-// planes, contiguous in B, into its plane buffer with one bulk copy per row, so no load goes through the
+// planes, contiguous in B, into its plane buffer with eight bulk copies (one per row, issued lane by lane,
+// kept a warp busy for thousands of cycles: 64^3 28.2 -> QNOW), so no load goes through the
 // LSU -- there a 16-byte load, whose lanes took half of 32 sectors in 8 or more lines, cost 24 L1 cycles,
 // 42 % of the L1 time at 64^3 -- and transforms both pairs in place between the same two barriers. Three
 // CTAs per SM at 64^3 hide each other's copies. Units of 16 bytes (one pair of one column) lie column by
 // column, pair by pair; a quarter-warp is 2 columns x 2 pairs x 2 blocks in y and 4 positions x 2 pairs in
-// z, 8 different banks with rows and blocks 4 mod 8 units apart. ms per 1e5 rotations (two smallest
+// z, 8 different banks with the strides below. ms per 1e5 rotations (two smallest
 // keys): 64^3 33.3 -> 28.8, 32^3 5.6 -> 4.4 against k_yz_pairs over the same quads; over plane pairs (FP32 x
 // pass, two shorter copies per row) the same scheme lost, 30.6 against 28.0 at 64^3.
 template <int N>
@@ -287,12 +287,11 @@ struct YzQuadShape {
   static constexpr int NZH = N / 2 + 1;
   static constexpr int T = N == 32 ? 160 : 288;
   static constexpr int CTAS = N == 32 ? 6 : 3;
-  static constexpr int UNITS = 2 * NZH;  // of a row
-  static constexpr int ROW = (UNITS + 3) / 8 * 8 + 4;
-  static constexpr int BLOCK = (N / 8) * ROW + 4;
-  static constexpr size_t SMEM = sizeof(float4) * ((N / 8) * 7 + 8 * BLOCK);
-  static_assert(ROW >= UNITS && ROW % 8 == 4 && BLOCK % 8 == 4, "row and block strides");
-  static_assert(ROW + UNITS >= 2 * N, "a row pair holds a line of both pairs");
+  static constexpr int ROW = 2 * NZH;              // 2 mod 8: a block of N / 8 rows as it lies in B
+  static constexpr int BLOCK = (N / 8) * ROW + 4;  // 4 mod 8
+  static constexpr size_t SMEM = sizeof(float2) * (N / 8) * 7 + sizeof(float4) * 8 * BLOCK;
+  static_assert(ROW % 8 == 2 && BLOCK % 8 == 4, "row and block strides");
+  static_assert(2 * ROW >= 2 * N, "a row pair holds a line of both pairs");
 };
 
 constexpr long kYzWaitLimit = 1l << 22;
@@ -303,8 +302,8 @@ __global__ void __launch_bounds__(YzQuadShape<N>::T, YzQuadShape<N>::CTAS) k_yz_
   constexpr int NZH = S::NZH, R1 = N / 8, T = S::T, NW = T / 32, ROW = S::ROW, BLOCK = S::BLOCK;
   static_assert(R1 <= 8 && b_quad_rots(N) == 1, "one second-stage group per lane, rotations apart");
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float4* tw = reinterpret_cast<float4*>(smem_raw);
-  float4* O = tw + R1 * 7;
+  float2* tw = reinterpret_cast<float2*>(smem_raw);
+  float4* O = reinterpret_cast<float4*>(tw + R1 * 7);
   __shared__ unsigned int s_bound;
   __shared__ __align__(8) uint64_t s_full;
   __shared__ int s_fail;
@@ -315,10 +314,7 @@ __global__ void __launch_bounds__(YzQuadShape<N>::T, YzQuadShape<N>::CTAS) k_yz_
   const int quads = (Wx + 3) / 4, npairs = (Wy + 1) / 2;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t full = (uint32_t)__cvta_generic_to_shared(&s_full);
-  for (int i = tid; i < R1 * 7; i += T) {
-    const float2 w = a.tw[(i / 7) * (i % 7 + 1)];
-    tw[i] = make_float4(w.x, w.x, w.y, w.y);
-  }
+  for (int i = tid; i < R1 * 7; i += T) tw[i] = a.tw[(i / 7) * (i % 7 + 1)];
   if (tid == 0) {
     s_bound = order_key(INFINITY);
     s_fail = 0;
@@ -333,17 +329,16 @@ __global__ void __launch_bounds__(YzQuadShape<N>::T, YzQuadShape<N>::CTAS) k_yz_
     const float2 x = unpk(v.x), y = unpk(v.y);
     *p = make_float4(x.x, x.y, y.x, y.y);
   };
-  // warp 0: the quad's rows into the plane buffer (row f = block f / R1, position f % R1)
+  // one thread: the quad's eight blocks into the plane buffer
   auto load_quad = [&](int p) {
-    constexpr uint32_t bytes = NZH * 32;
-    if (lane == 0)
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%1], %0;" ::"r"(bytes * N), "r"(full) : "memory");
-    __syncwarp();
+    constexpr uint32_t bytes = R1 * NZH * 32;
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%1], %0;" ::"r"(bytes * 8), "r"(full) : "memory");
     const float4* src = reinterpret_cast<const float4*>(a.B) + b_quad_index<N>(r, 0) + (size_t)p * (N * NZH * 2);
-    for (int f = lane; f < N; f += 32)
+#pragma unroll 1
+    for (int b = 0; b < 8; ++b)
       asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                       (uint32_t)__cvta_generic_to_shared(O + (f / R1) * BLOCK + (f % R1) * ROW)),
-                   "l"(src + (size_t)f * (NZH * 2)), "r"(bytes), "r"(full)
+                       (uint32_t)__cvta_generic_to_shared(O + b * BLOCK)),
+                   "l"(src + b * (R1 * ROW)), "r"(bytes), "r"(full)
                    : "memory");
   };
   auto wait_quad = [&](uint32_t parity) {
@@ -365,13 +360,15 @@ __global__ void __launch_bounds__(YzQuadShape<N>::T, YzQuadShape<N>::CTAS) k_yz_
     *(volatile int*)&s_fail = 1;
   };
   const int q = lane & 1;                          // the lane's pair of the quad
-  const int ty = lane >> 2;                        // y: block or group; columns 2u, 2u + 1 of unit u
+  const int ty = lane >> 2;                        // y: block; columns 2u, 2u + 1 of unit u
+  // and group: the quarter-warp's two groups 2 rows, 4 units mod 8, apart
+  const int np = (ty & 4) | ((ty & 1) << 1) | ((ty >> 1) & 1);
   const int t = (lane >> 1) & 7, g2 = lane >> 4;   // z: place in the line; row pairs 2w, 2w + 1 of unit w
   constexpr int SW = R1 - 1;  // swizzle of a line's positions b R1 + m -> b R1 + (m ^ (b & SW))
   const float inv = 1.0f / (float)((double)N * N * N);
   unsigned long long best = ~0ull, best2 = ~0ull;
   __syncthreads();
-  if (warp == 0 && part < quads) load_quad(part);
+  if (tid == 0 && part < quads) load_quad(part);
   uint32_t parity = 0;
 #pragma unroll 1
   for (int p = part; p < quads; p += parts, parity ^= 1u) {
@@ -391,14 +388,14 @@ __global__ void __launch_bounds__(YzQuadShape<N>::T, YzQuadShape<N>::CTAS) k_yz_
         for (int j = 0; j < R1; ++j) st(col + ty * BLOCK + j * ROW, v[j]);
       }
       __syncwarp();
-      if (has_col && ty < R1) {
+      if (has_col && np < R1) {
         cpair v[8];
 #pragma unroll
-        for (int b = 0; b < 8; ++b) v[b] = ld(col + b * BLOCK + ty * ROW);
-        yz_twiddle<N>(v, tw, ty);
+        for (int b = 0; b < 8; ++b) v[b] = ld(col + b * BLOCK + np * ROW);
+        yz_twiddle<N>(v, tw, np);
         PairRadix<8, +1>::run(v);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) st(col + j * BLOCK + ty * ROW, v[j]);
+        for (int j = 0; j < 8; ++j) st(col + j * BLOCK + np * ROW, v[j]);
       }
     }
     __syncthreads();
@@ -442,7 +439,7 @@ __global__ void __launch_bounds__(YzQuadShape<N>::T, YzQuadShape<N>::CTAS) k_yz_
     // the next quad's copies (async proxy) follow every read and write of this one
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
-    if (warp == 0 && p + parts < quads) load_quad(p + parts);
+    if (tid == 0 && p + parts < quads) load_quad(p + parts);
   }
   yz_store<N, NW, TOP2>(a, r, part, O, best, best2);
   if (tid == 0 && s_fail) {

@@ -1,17 +1,19 @@
-"""The inverse (y,z) kernel over whole plane quads (one-column Hankel x pass, n <= 64) against the
-single-plane kernel: the same bits, with one quad per CTA (few rotations) and several (many), for
-windows that leave 1, 2, 3 or 4 planes in the last quad, with and without the two smallest keys."""
+"""The inverse (y,z) kernels with bulk copies (two plane pairs at once at n <= 64, one FP32 pair
+above) against the single-plane kernel: the same bits, with one turn per CTA (few rotations) and
+several (many), for windows that leave 1, 2, 3 or 4 planes in the last quad, with and without the two
+smallest keys."""
 import numpy as np
 import pytest
 
-from cdocker_b200 import CDK_FORM_BF16X3, CDK_FORM_FP16X2, Receptor
+from cdocker_b200 import CDK_FORM_BF16X3, CDK_FORM_FP16X2, CDK_FORM_FP32, Receptor
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("form", [CDK_FORM_FP16X2, CDK_FORM_BF16X3])
+@pytest.mark.parametrize("form", [CDK_FORM_FP32, CDK_FORM_FP16X2, CDK_FORM_BF16X3])
 @pytest.mark.parametrize("tie_break", [True, False])
-@pytest.mark.parametrize("n,rots,atoms", [(32, 2, 5), (32, 2500, 9), (64, 3, 40), (64, 900, 14)])
+@pytest.mark.parametrize("n,rots,atoms", [(32, 2, 5), (32, 2500, 9), (64, 3, 40), (64, 900, 14),
+                                          (96, 1, 9), (96, 250, 14), (128, 160, 9)])
 def test_same_bits_as_single_planes(form, tie_break, n, rots, atoms):
     rng = np.random.default_rng([n, rots, atoms])
     grids = rng.normal(size=(3, n, n, n)).astype(np.float32)

@@ -633,7 +633,7 @@ int check_errors_after(cdk_ctx* c, cudaStream_t s) {
                            cudaMemcpyDeviceToHost, s));
   CDK_CUDA(cudaStreamSynchronize(s));
   if (c->h_misc[3] != 0) {
-    set_error("a bounded device wait (tensor-core commit) gave up; results are invalid");
+    set_error("a bounded device wait (copies, tensor-core commit) gave up; results are invalid");
     return CDK_ERR_CUDA;
   }
   float ms = 0.f;

@@ -70,7 +70,7 @@ int scratch_for_device(int dev, void** out) {
 size_t up256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // misc words at the head of the array: [0] diameter bits, [1] input flags, [2] overflow
-// count, [4..7] work counters (two u64)
+// count, [3] a device wait gave up, [4..7] work counters (two u64)
 constexpr size_t kMiscBytes = 256;
 
 __global__ void k_na_check(int nAtom, int nConf, const float* coor, const int* slot, int K,
@@ -251,8 +251,12 @@ extern "C" int cdk_search_device_noalloc(cdk_ctx* ctx, int nAtom, int nConf,
     NA_CUDA(launch_yz_inv_argmin(a, s));
     NA_CUDA(launch_finalize(a, s));
   }
-  NA_CUDA(cudaMemcpyAsync(v.h_misc + 2, misc + 2, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
+  NA_CUDA(cudaMemcpyAsync(v.h_misc + 2, misc + 2, 2 * sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
   NA_CUDA(cudaStreamSynchronize(s));
+  if (v.h_misc[3] != 0) {
+    set_error("a bounded device wait gave up; results are invalid");
+    return CDK_ERR_CUDA;
+  }
   if (v.h_misc[2] != 0) {
     set_error(std::to_string(v.h_misc[2]) +
               " rotation(s) overflowed the planned ligand box; results for them are invalid");

@@ -242,7 +242,7 @@ void retire(cdk_server* s, WaveSlot& w, int slot) {
       else if (se != cudaSuccess)
         fail_request(r, CDK_ERR_CUDA, std::string("its wave did not complete: ") + cudaGetErrorString(se));
       else if (st[1] != 0)
-        fail_request(r, CDK_ERR_CUDA, "a bounded device wait (tensor-core commit) gave up in its wave; "
+        fail_request(r, CDK_ERR_CUDA, "a bounded device wait (copies, tensor-core commit) gave up in its wave; "
                                       "results are invalid");
       else if (st[0] != 0 || st[2] != 0)
         r->scan = true;

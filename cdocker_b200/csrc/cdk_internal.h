@@ -85,8 +85,8 @@ struct WaveArgs {
                              // (nrot rounded up to a multiple of R; bgroup 4, bcol 1); 0: not
                              // paired. Read by launch_yz_pairs only
   int key_slots;             // key pairs per rotation in keys2 (0: one per window plane)
-  int yz_block_stages;       // inverse (y,z) kernel: 0 by grid size (block stages at n <= 64,
-                             // octets at n >= 96), 1 block stages, 2 octets
+  int yz_block_stages;       // inverse (y,z) kernel: 0 over plane pairs (bpairs; other B layouts:
+                             // block stages at n <= 64, octets at n >= 96), 1 block stages, 2 octets
   unsigned long long* keys;  // [nrot]
   unsigned long long* keys2; // precision forms' near-tie break: [nrot][n][2] the two smallest
                              // keys of every window plane (null: not kept)
@@ -102,7 +102,8 @@ struct WaveArgs {
   int chunk;                 // rotations per CTA in the x pass (0 = default)
   int* fault;                // set when a bounded device wait gave up
   const int* kyof;           // [n] natural frequency at each digit-reversed position; when set
-                             // (and ligands have <= 96 atoms) planes are evaluated directly
+                             // (and ligands have <= 96 atoms, split-BF16 rows 128) planes are
+                             // evaluated directly
   int f16;                   // split-FP16 form: the plane kernel writes FP16 rows (8 per rotation
                              // and channel: [chunk][re, im]) of the planes times lscale[k]
   float lscale[KMAX];        // split-FP16 form: 2^sigma_k per channel (a power of two, exact)
@@ -145,7 +146,7 @@ inline bool hankel_tiled(int reserved5) { return !(reserved5 & 32) && tensor_map
 // whose planes lie a rotation's B apart: 1.1 MB at 64^3, but 3.6 MB at 96^3 and 8.5 MB at 128^3, a page
 // of their own each. Two rotations per 64-byte run halve the pages and lines of a store (x pass 128^3,
 // 1e5 rotations: 562 -> 390 ms, yz 362 -> 397; 96^3: 215 -> 184, 132 -> 142); at 64^3 the yz pass lost
-// what the x pass gained (46.8 for 48.2 ms, 34.3 for 31.7). Four or more gave the x pass nothing further.
+// what the x pass gained (46.8 for 48.2 ms, 34.3 for 31.7), and its bulk copies bring whole quads. Four or more gave the x pass nothing further.
 constexpr int b_quad_rots(int n) { return n >= 96 ? 2 : 1; }
 // rotations a wave's window planes (WaveArgs.B) are allocated for
 inline size_t b_rotations(long nrot) { return (size_t)((nrot + 1) & ~1L); }

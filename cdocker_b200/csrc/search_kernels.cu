@@ -3,16 +3,17 @@
 // One wave of rotations runs five kernels, all on one stream:
 //   prep          rotate atoms (reference op order, no contraction), bounding box, windows,
 //                 per-channel x-plane ranges          (src/Rotate.cpp, GetMin/MaxCoors.cpp)
-//   spread_yz     per (rotation, channel, x plane): spread the atoms that touch the plane
-//                 into shared memory (trilinear weights in FillLigandGrid's arithmetic), then
-//                 the 2-D real-to-complex FFT over (y,z) -> A      (src/FillLigandGrid.cpp)
+//   spread_yz     per rotation (up to 96 atoms): the (y,z) spectra of the planes its atoms touch as
+//                 sums of separable spectra of their trilinear weights -> A; larger ligands, per
+//                 (rotation, channel, x plane): spread the atoms into shared memory (FillLigandGrid's
+//                 arithmetic), then the 2-D real-to-complex FFT   (src/FillLigandGrid.cpp)
 //   xpass         (fp32_xpass.cu) per spectral column tile: FFT along x of every channel, the conjugate
 //                 product with the resident receptor spectra summed over channels, and the
 //                 inverse FFT along x, keeping only the translation window -> B
 //                                                       (src/kernel.cu ConjMult + SumGrids)
-//   yz_inv_argmin per (rotation, x in window): inverse FFT over y, complex-to-real over z,
-//                 min / first argmin over the window, folded into one 64-bit key per rotation
-//                                         (src/TranRotaConfSearchNoMini.cu:429-464)
+//   yz_inv_argmin (yz_pairs.cu) per (rotation, planes x, x + 1 in window): inverse FFT over y, complex-
+//                 to-real over z, min / first argmin over the window, folded into one 64-bit key per
+//                 rotation                (src/TranRotaConfSearchNoMini.cu:429-464)
 //   finalize      keys -> minE, (i,j,k)
 // The energy grid never leaves shared memory. Spectra stay in the digit-reversed order the
 // in-place FFT stages produce; the receptor spectra are computed by the same stages, so
@@ -1401,9 +1402,10 @@ cudaError_t launch_spread_yz_t(const WaveArgs& a, cudaStream_t s) {
 
 template <int N>
 cudaError_t launch_yz_inv_t(const WaveArgs& a, cudaStream_t s) {
-  // octet kernel at n >= 96 (measured 2.1x faster than block stages at 128^3, 1.05x at 96^3);
-  // block stages at n <= 64 (the packed rows alias the plane there, 8 CTAs per SM: 1.6x faster
-  // than the octets at 64^3); yz_block_stages: 1 forces block stages, 2 forces octets
+  // the single-plane kernels: plain and column-pair B (x passes on request), and on request. Octets at
+  // n >= 96 (measured 2.1x faster than block stages at 128^3, 1.05x at 96^3); block stages at n <= 64
+  // (the packed rows alias the plane there, 8 CTAs per SM: 1.6x faster than the octets at 64^3);
+  // yz_block_stages: 1 forces block stages, 2 forces octets
   const bool octet = a.yz_block_stages == 2 || (a.yz_block_stages == 0 && N >= 96);
   // the B layout as a template argument (kBAny reads it at run time)
   const int bl = b_layout(a);

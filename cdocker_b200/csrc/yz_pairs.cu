@@ -23,7 +23,7 @@
 // Measured on a B200, inverse pass, against the single-plane kernels of before (ms per 1e5 rotations): over
 // quads with the two smallest keys 64^3 42.9 -> 25.2, 96^3 259 -> 130, 128^3 672 -> 350; over plane pairs 64^3
 // 30.2 -> 23.2, 96^3 221 -> 119, 128^3 526 -> 306 (96^3 1.25 -> 1.19 and 128^3 3.21 -> 3.06 ms per 1,000 by the
-// bulk copies). What bounds it now is the shared-memory data path (60 % at 64^3) beside the CTA barriers;
+// bulk copies). What bounds it now is the shared-memory data path (70 % at 64^3) beside the CTA barriers;
 // at 128^3, where the plane buffer allows one CTA per SM, the barriers and the load latency.
 //
 // The smallest key (two smallest: TOP2) is carried over the CTA's planes and reduced once at its

@@ -58,8 +58,8 @@ typedef struct cdk_opts {
                           [1] bit 0: spread planes through the radix FFT instead of the direct
                           separable evaluation; bit 1: the inverse (y,z) kernel with
                           block-wide radix stages at every n; bit 2: the one with warp-local
-                          line transforms at every n (default: block stages at n <= 64,
-                          warp-local lines at n >= 96); [2] = 1: autotune the x pass on the first wave
+                          line transforms at every n (default: two planes at a time where
+                          the x pass writes plane pairs or quads); [2] = 1: autotune the x pass on the first wave
                           of each new ligand box; [3] precision-form x pass: 0 = automatic
                           (ligands <= 96 atoms, box <= 32 planes: tcgen05 with the Hankel
                           operator resident in shared memory; split-BF16 ligands above 128
@@ -292,7 +292,7 @@ int cdk_server_destroy(cdk_server* s);
  * [0] kernel launches, [1] waves, [2] rotations, [3] device ms of the search (events on the
  * search stream), [4] planned ligand box edge, [5] rotations per wave, [6] (y,z) planes the
  * spread kernel transformed, [7] window planes the x pass wrote, [8..12] device ms per kernel
- * kind (prep, spread_yz, xpass, yz_inv_argmin, finalize) when the context was created with
+ * kind (prep, spread_yz, xpass, yz_inv_argmin with the near-tie break, finalize with the top poses) when the context was created with
  * opts.reserved[0] = 1 (events around every launch), else 0; [13] x-pass column tile (FP32 form: opts.col_tile, 8 when 0),
  * [14] x-pass rotations per CTA, [15] graph state (0 off, 1 shape seen, 2 replaying),
  * [16] x-pass kind (0 FP32 radix, 1 mma.sync, 2 tcgen05 for split-BF16 ligands above 96 atoms:

@@ -146,7 +146,8 @@ inline bool hankel_tiled(int reserved5) { return !(reserved5 & 32) && tensor_map
 // whose planes lie a rotation's B apart: 1.1 MB at 64^3, but 3.6 MB at 96^3 and 8.5 MB at 128^3, a page
 // of their own each. Two rotations per 64-byte run halve the pages and lines of a store (x pass 128^3,
 // 1e5 rotations: 562 -> 390 ms, yz 362 -> 397; 96^3: 215 -> 184, 132 -> 142); at 64^3 the yz pass lost
-// what the x pass gained (46.8 for 48.2 ms, 34.3 for 31.7), and its bulk copies bring whole quads. Four or more gave the x pass nothing further.
+// what the x pass gained (46.8 for 48.2 ms, 34.3 for 31.7), and its bulk copies bring whole quads. Four
+// or more gave the x pass nothing further.
 constexpr int b_quad_rots(int n) { return n >= 96 ? 2 : 1; }
 // rotations a wave's window planes (WaveArgs.B) are allocated for
 inline size_t b_rotations(long nrot) { return (size_t)((nrot + 1) & ~1L); }

@@ -398,8 +398,10 @@ void worker_loop(cdk_server* s) {
     a.Lb = lb;
     a.atom_cap = cap;
     a.rots = w.d_rots;
-    // the same x-pass choice as a plain search on the context (results alone and in the mix
-    // stay identical): streamed tiles at 64^3 where they apply, the Hankel kernel elsewhere
+    // tensor-core waves take the x pass of a plain search on the context (results alone and in the mix
+    // stay identical): streamed tiles at 64^3 on request, the Hankel kernel elsewhere. A wave that holds
+    // a ligand above 96 atoms or a box above 32 planes runs the FP32 x pass in every form, for all its
+    // requests: theirs are then the FP32 form's energies
     HankelPlan hp{};
     const bool tile_wave = s->streamed && s->v.top != nullptr && use_stream_tiles(s->v.tc_variant) &&
                            stream_supported(n, lb) && direct_planes(a);
@@ -411,7 +413,9 @@ void worker_loop(cdk_server* s) {
     a.f16 = (tc_wave && f16) ? 1 : 0;
     a.bgroup = tc_wave ? stream_bgroup() : 1;
     a.bcol = 0;
-    a.bpairs = tc_wave ? 0 : 2;  // the FP32 x pass writes plane pairs
+    // the FP32 x pass writes plane pairs, but for the inverse kernels that keep the near-tie break's two
+    // smallest keys the plain layout: over plane pairs there is none with them
+    a.bpairs = tc_wave || a.keys2 ? 0 : 2;
     if (tc_wave && !tile_wave) hankel_b_layout(hp, a);
     a.key_slots = a.bpairs ? yz_pairs_key_slots(a) : 0;
     if (le == cudaSuccess) {

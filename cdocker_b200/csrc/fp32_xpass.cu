@@ -526,7 +526,9 @@ bool xp_plan(const WaveArgs& a, XpPlan* p) {
 template <int N, int JM>
 cudaError_t launch_xp_jm(const WaveArgs& a, const XpPlan& p, cudaStream_t s) {
   auto kern = k_xpass_pairs<N, JM>;
-  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
+  // the most that any shape asks for and not this launch's: the attribute is the process's, and another
+  // thread's smaller shape, set between this call and the launch, would refuse it
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kXpSmemCap);
   if (e != cudaSuccess) return e;
   constexpr int NCOL = N * (N / 2 + 1);
   kern<<<dim3(NCOL / XP_COLS, (a.nrot + p.chunk - 1) / p.chunk), 128 * p.G, p.smem, s>>>(a, xp_twiddles<N>(), p.chunk,

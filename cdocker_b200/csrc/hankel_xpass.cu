@@ -794,7 +794,8 @@ cudaError_t launch_hx(const WaveArgs& a, const float2* pt, const HxScale& sc, in
                       size_t smem, int ctas_per_sm, cudaStream_t s) {
   constexpr int NCOL = N * (N / 2 + 1);
   auto kern = k_xpass_hankel<N, COLS, F16>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // the most that any plan asks for: the attribute is the process's (other threads' plans)
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCap);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return e;

@@ -1379,17 +1379,20 @@ template <int N>
 cudaError_t launch_spread_yz_t(const WaveArgs& a, cudaStream_t s) {
   const int cap = a.atom_cap > 0 ? a.atom_cap : a.max_atoms;
   if (a.kyof && cap <= direct_max_atoms(!a.lop ? kRowsNone : a.f16 ? kRowsF16 : kRowsBf16)) {
-    auto launch = [&](auto kern, size_t sm, int threads) {
-      const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    auto launch = [&](auto kern, auto shape, int rows) {
+      // room for the largest ligand whatever this one's atoms: the attribute is the process's, and another
+      // thread's smaller ligand, set between this call and the launch, would refuse it
+      const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)shape.smem(direct_max_atoms(rows)));
       if (e != cudaSuccess) return e;
       // parts of a rotation's items: enough CTAs for small waves (each part repeats the tables)
       const int parts = std::max(1, std::min(a.K, (148 * 6 + a.nrot - 1) / a.nrot));
-      kern<<<dim3(parts, a.nrot), threads, sm, s>>>(a, a.kyof, cap);
+      kern<<<dim3(parts, a.nrot), shape.T, shape.smem(cap), s>>>(a, a.kyof, cap);
       return cudaGetLastError();
     };
-    if (!a.lop) return launch(k_spread_yz_direct<N, kRowsNone>, DirectShape<N, kRowsNone>::smem(cap), DirectShape<N, kRowsNone>::T);
-    if (a.f16) return launch(k_spread_yz_direct<N, kRowsF16>, DirectShape<N, kRowsF16>::smem(cap), DirectShape<N, kRowsF16>::T);
-    return launch(k_spread_yz_direct<N, kRowsBf16>, DirectShape<N, kRowsBf16>::smem(cap), DirectShape<N, kRowsBf16>::T);
+    if (!a.lop) return launch(k_spread_yz_direct<N, kRowsNone>, DirectShape<N, kRowsNone>{}, kRowsNone);
+    if (a.f16) return launch(k_spread_yz_direct<N, kRowsF16>, DirectShape<N, kRowsF16>{}, kRowsF16);
+    return launch(k_spread_yz_direct<N, kRowsBf16>, DirectShape<N, kRowsBf16>{}, kRowsBf16);
   }
   if (a.lop) return cudaErrorInvalidValue;  // the FFT plane path writes A only
   const size_t sm = plane_smem<N>();

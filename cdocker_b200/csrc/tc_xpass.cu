@@ -260,7 +260,8 @@ cudaError_t launch_tc_t(const WaveArgs& a, const float2* pt, cudaStream_t s) {
   constexpr int NCOL = N * (N / 2 + 1);
   const int Lp = (a.Lb + 7) & ~7;
   const size_t sm = xpass_tc_smem_bytes(N, a.K, a.Lb);
-  cudaError_t e = cudaFuncSetAttribute(k_xpass_tc<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  // the most that any box asks for: the attribute is the process's (other threads' boxes)
+  cudaError_t e = cudaFuncSetAttribute(k_xpass_tc<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
   if (e != cudaSuccess) return e;
   const int per = a.chunk > 0 ? ((a.chunk + 15) / 16) * 16 : 64;
   const int chunks = (a.nrot + per - 1) / per;

@@ -379,7 +379,9 @@ cudaError_t launch_xpass_umma(const WaveArgs& a, const float2* pt, cudaStream_t 
   if (!umma_supported(a.n, a.Lb)) return cudaErrorInvalidValue;
   const int Lp = (a.Lb + 7) & ~7;
   const size_t sm = xpass_umma_smem_bytes(a.Lb);
-  cudaError_t e = cudaFuncSetAttribute(k_xpass_umma64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  // the largest box's: the attribute is the process's (other threads' boxes)
+  cudaError_t e = cudaFuncSetAttribute(k_xpass_umma64, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)xpass_umma_smem_bytes(32));
   if (e != cudaSuccess) return e;
   constexpr int NCOL = 64 * 33;
   dim3 grid(NCOL / UM_CT, (a.nrot + UM_R - 1) / UM_R);

@@ -35,6 +35,7 @@
 #include <algorithm>
 
 #include "cdk_internal.h"
+#include "copy_turns.cuh"
 #include "pair_fft.cuh"
 #include "window_keys.cuh"
 
@@ -108,6 +109,21 @@ __device__ __forceinline__ void yz_load(float4* dst, const float4* src, uint32_t
   }
 }
 
+// The operations of copy_turns from a kernel's lambdas
+template <class Load, class Wait, class Columns, class Failed, class Rows, class Drain>
+struct YzTurns {
+  Load load;
+  Wait wait;
+  Columns columns;
+  Failed failed;
+  Rows rows;
+  Drain drain;
+};
+template <class... F>
+__device__ __forceinline__ YzTurns<F...> yz_turns(F... f) {
+  return {f...};
+}
+
 // min that keeps a NaN
 __device__ __forceinline__ float min_nan(float a, float b) {
   float r;
@@ -171,6 +187,14 @@ __device__ __forceinline__ void yz_keep(const cpair* u, bool on, int np, int x, 
       }
     }
   }
+}
+
+// A CTA whose copies did not come: reports it and leaves no keys
+template <int N, bool TOP2>
+__device__ __forceinline__ void yz_give_up(const WaveArgs& a, int r, int part) {
+  if (threadIdx.x != 0) return;
+  atomicOr(a.fault, 1);
+  if constexpr (TOP2) a.keys2[((size_t)r * N + part) * 2] = a.keys2[((size_t)r * N + part) * 2 + 1] = ~0ull;
 }
 
 // The CTA's smallest keys, reduced in the plane buffer (free by now) and stored
@@ -249,15 +273,19 @@ __global__ void __launch_bounds__(YzShape<N, QUADS>::T, YzShape<N, QUADS>::CTAS)
   const int sw = R1 % 8 == 0 ? t : t >> 1;  // swizzle of a line's positions t R1 + m -> t R1 + (m ^ sw)
   const float inv = 1.0f / (float)((double)N * N * N);
   unsigned long long best = ~0ull, best2 = ~0ull;
-  auto load_pair = [&](int p) {  // plane pairs, one thread: the eight blocks into the plane buffer
-    yz_load<1>(O, src0 + (size_t)p * NCOL, R1 * NZH * 16, BLOCK, 0, R1 * NZH, 0, full);
+  // plane pairs, one thread: the eight blocks into the plane buffer
+  auto load = [&](int p) {
+    if (!QUADS && tid == 0) yz_load<1>(O, src0 + (size_t)p * NCOL, R1 * NZH * 16, BLOCK, 0, R1 * NZH, 0, full);
   };
-  uint32_t parity = 0;
-  __syncthreads();
-  if (!QUADS && tid == 0 && part < pairs) load_pair(part);
-#pragma unroll 1
-  for (int p = part; p < pairs; p += parts, parity ^= 1u) {
+  auto wait = [&](uint32_t parity) {
     if constexpr (!QUADS) yz_wait(full, parity, &s_fail);
+  };
+  auto failed = [&] { return !QUADS && *(volatile int*)&s_fail != 0; };
+  auto drain = [&](uint32_t parity) {
+    int gave_up = 0;
+    if (!QUADS && tid == 0) yz_wait(full, parity, &gave_up);
+  };
+  auto columns = [&](int p) {
     // y of column gy: first stage (radix R1, no twiddles) over block ty's positions
     if (has_col) {
       cpair v[R1];
@@ -290,6 +318,8 @@ __global__ void __launch_bounds__(YzShape<N, QUADS>::T, YzShape<N, QUADS>::CTAS)
       }
     }
     __syncthreads();
+  };
+  auto rows = [&](int p) {
     // z of row pair g: rows (2g, 2g + 1) as one complex line with its Hermitian extension
     if ((g & ~3) < npairs) {  // warp-uniform: one of the warp's octets has a row pair
       const bool act = g < npairs;
@@ -332,14 +362,11 @@ __global__ void __launch_bounds__(YzShape<N, QUADS>::T, YzShape<N, QUADS>::CTAS)
     // the next pair's copies (async proxy) follow every read and write of this one
     if constexpr (!QUADS) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
-    if (!QUADS && tid == 0 && p + parts < pairs) load_pair(p + parts);
-  }
-  yz_store<N, T / 32, TOP2>(a, r, part, O, best, best2);
-  if (!QUADS && tid == 0 && s_fail) {
-    atomicOr(a.fault, 1);
-    s_fail = 0;
-    yz_wait(full, parity ^ 1u, &s_fail);  // a copy still in flight lands before the CTA leaves
-  }
+  };
+  __syncthreads();
+  auto turns = yz_turns(load, wait, columns, failed, rows, drain);
+  if (copy_turns(part, parts, pairs, turns)) yz_store<N, T / 32, TOP2>(a, r, part, O, best, best2);
+  else yz_give_up<N, TOP2>(a, r, part);
 }
 
 // Two plane pairs at once (n <= 64): a CTA brings them into its plane buffer with bulk copies, so no load
@@ -404,10 +431,16 @@ __global__ void __launch_bounds__(YzTwoShape<N, QUADS>::T, YzTwoShape<N, QUADS>:
     *p = make_float4(x.x, x.y, y.x, y.y);
   };
   // one thread: the eight blocks of both pairs into the plane buffer
-  auto load_quad = [&](int p) {
+  auto load = [&](int p) {
     constexpr int COPIES = QUADS ? 1 : 2;  // per block
     const float4* src = reinterpret_cast<const float4*>(a.B) + ((size_t)r * (N / 4) + p) * (N * NZH * 2);
-    yz_load<COPIES>(O, src, R1 * NZH * 32 / COPIES, BLOCK, S::PAIR, R1 * ROW, N * NZH, full);
+    if (tid == 0) yz_load<COPIES>(O, src, R1 * NZH * 32 / COPIES, BLOCK, S::PAIR, R1 * ROW, N * NZH, full);
+  };
+  auto wait = [&](uint32_t parity) { yz_wait(full, parity, &s_fail); };
+  auto failed = [&] { return *(volatile int*)&s_fail != 0; };
+  auto drain = [&](uint32_t parity) {
+    int gave_up = 0;
+    if (tid == 0) yz_wait(full, parity, &gave_up);
   };
   const int q = lane & 1;                          // the lane's pair of the quad
   const int ty = lane >> 2;                        // y: block; columns 2u, 2u + 1 of unit u
@@ -417,12 +450,7 @@ __global__ void __launch_bounds__(YzTwoShape<N, QUADS>::T, YzTwoShape<N, QUADS>:
   constexpr int SW = R1 - 1;  // swizzle of a line's positions b R1 + m -> b R1 + (m ^ (b & SW))
   const float inv = 1.0f / (float)((double)N * N * N);
   unsigned long long best = ~0ull, best2 = ~0ull;
-  __syncthreads();
-  if (tid == 0 && part < quads) load_quad(part);
-  uint32_t parity = 0;
-#pragma unroll 1
-  for (int p = part; p < quads; p += parts, parity ^= 1u) {
-    yz_wait(full, parity, &s_fail);
+  auto columns = [&](int p) {
     // y: both stages of columns 2u, 2u + 1 and both pairs by one warp
 #pragma unroll 1
     for (int u = warp; u < (NZH + 1) / 2; u += NW) {
@@ -449,6 +477,8 @@ __global__ void __launch_bounds__(YzTwoShape<N, QUADS>::T, YzTwoShape<N, QUADS>:
       }
     }
     __syncthreads();
+  };
+  auto rows = [&](int p) {
     // z: rows (2g, 2g + 1) as one complex line with its Hermitian extension
     const int x = 4 * p + 2 * q;
     const bool pair = x < Wx, plane1 = x + 1 < Wx;
@@ -489,14 +519,11 @@ __global__ void __launch_bounds__(YzTwoShape<N, QUADS>::T, YzTwoShape<N, QUADS>:
     // the next quad's copies (async proxy) follow every read and write of this one
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
-    if (tid == 0 && p + parts < quads) load_quad(p + parts);
-  }
-  yz_store<N, NW, TOP2>(a, r, part, O, best, best2);
-  if (tid == 0 && s_fail) {
-    atomicOr(a.fault, 1);
-    s_fail = 0;
-    yz_wait(full, parity ^ 1u, &s_fail);  // a copy still in flight lands before the CTA leaves
-  }
+  };
+  __syncthreads();
+  auto turns = yz_turns(load, wait, columns, failed, rows, drain);
+  if (copy_turns(part, parts, quads, turns)) yz_store<N, NW, TOP2>(a, r, part, O, best, best2);
+  else yz_give_up<N, TOP2>(a, r, part);
 }
 
 // CTAs per rotation: about 16 rounds of CTAs over the device, so that the last one costs little,

@@ -26,6 +26,7 @@
 // All double arithmetic uses explicit round-to-nearest intrinsics (no contraction), sqrt and
 // division are IEEE, and every sum runs in atom order: the RMSDs are bit-identical to a host
 // double-precision evaluation of the same recipe without fused multiply-adds.
+#include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -279,11 +280,35 @@ std::vector<int> selected_atoms(int nAtom, const unsigned char* mask) {
 // destroyed: no CUDA call runs while the process exits.
 constexpr size_t CL_KEEP = (size_t)32 << 20;
 constexpr size_t CL_IDLE = 2;
+
+// The driver's number of the allocation that holds p: unique in the process, never used again (0: none).
+// A device reset takes a kept space's memory and stream away, and a later allocation, the caller's own,
+// may get the same address (seen on a B200: the first allocation after a reset did), so a kept space
+// is known by this number and not by its address.
+unsigned long long buffer_id(const void* p) {
+  static const PFN_cuPointerGetAttribute_v4000 attribute = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q{};
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      f = nullptr;
+    return reinterpret_cast<PFN_cuPointerGetAttribute_v4000>(f);
+  }();
+  unsigned long long id = 0;
+  if (!attribute || !p ||
+      attribute(&id, CU_POINTER_ATTRIBUTE_BUFFER_ID, reinterpret_cast<CUdeviceptr>(p)) != CUDA_SUCCESS)
+    return 0;
+  return id;
+}
+
 struct ClusterSpace {
   int dev = -1;
   void* base = nullptr;
   size_t cap = 0;
   cudaStream_t s = nullptr;
+  unsigned long long id = 0;  // of base
+  // its memory, and so its context and stream, are still its own
+  bool alive() const { return id != 0 && buffer_id(base) == id; }
   void drop() {
     int d = 0;
     const bool moved = dev >= 0 && cudaGetDevice(&d) == cudaSuccess && d != dev;
@@ -291,9 +316,7 @@ struct ClusterSpace {
     if (base) cudaFree(base);
     if (s) cudaStreamDestroy(s);
     if (moved) cudaSetDevice(d);
-    base = nullptr;
-    s = nullptr;
-    cap = 0;
+    *this = ClusterSpace{};
   }
 };
 struct ClusterIdle {
@@ -327,13 +350,7 @@ struct ClusterBuffers {
           idle.spaces.erase(idle.spaces.begin() + i);
         }
     }
-    if (space.base) {
-      cudaPointerAttributes at{};
-      if (cudaPointerGetAttributes(&at, space.base) != cudaSuccess || at.type != cudaMemoryTypeDevice) {
-        (void)cudaGetLastError();
-        space = ClusterSpace{};  // the device was reset: memory and stream are gone
-      }
-    }
+    if (space.base && !space.alive()) space = ClusterSpace{};  // the device was reset: nothing to give back
     space.dev = d;
     if (!space.s && (e = cudaStreamCreateWithFlags(&space.s, cudaStreamNonBlocking)) != cudaSuccess) {
       space.s = nullptr;
@@ -344,17 +361,19 @@ struct ClusterBuffers {
       if (space.base) cudaFree(space.base);
       space.base = nullptr;
       space.cap = 0;
+      space.id = 0;
       if ((e = cudaMalloc(&space.base, bytes)) != cudaSuccess) {
         space.base = nullptr;
         return e;
       }
       space.cap = bytes;
+      space.id = buffer_id(space.base);
     }
     return cudaSuccess;
   }
   ~ClusterBuffers() {
     if (!space.s) return;
-    if (cudaStreamSynchronize(space.s) == cudaSuccess && space.base && space.cap <= CL_KEEP) {
+    if (cudaStreamSynchronize(space.s) == cudaSuccess && space.id != 0 && space.cap <= CL_KEEP) {
       ClusterIdle& idle = cluster_idle();
       std::lock_guard<std::mutex> lk(idle.mu);
       if (idle.spaces.size() < CL_IDLE) {
@@ -433,7 +452,8 @@ int check_inputs(int nConf, int nAtom, const double* coor, const unsigned char* 
 void cluster_release() {
   ClusterIdle& idle = cluster_idle();
   std::lock_guard<std::mutex> lk(idle.mu);
-  for (ClusterSpace& sp : idle.spaces) sp.drop();
+  for (ClusterSpace& sp : idle.spaces)
+    if (sp.alive()) sp.drop();
   idle.spaces.clear();
 }
 

@@ -106,6 +106,7 @@ SIGNATURES = {
     "cdk_cluster_conformers": (C.c_int, [C.c_int, C.c_int, _dp, _dp, _vp, C.c_double, C.c_int,
                                          _ip, _ip]),
     "cdk_pair_rmsd": (C.c_int, [C.c_int, C.c_int, _dp, _vp, _dp]),
+    "cdk_cluster_release": (C.c_int, []),
 }
 
 _lib = None

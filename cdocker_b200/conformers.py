@@ -55,3 +55,9 @@ def pair_rmsd(coords, atom_mask=None) -> np.ndarray:
     _lib.check(_lib.lib().cdk_pair_rmsd(n_conf, n_atoms, coords.ctypes.data_as(_dp), mptr,
                                         out.ctypes.data_as(_dp)))
     return out
+
+
+def release_workspaces() -> int:
+    """Gives back the device memory that the two calls above keep between calls (at most two
+    workspaces of 32 MB; closing a Receptor gives back its device's). Returns how many there were."""
+    return int(_lib.lib().cdk_cluster_release())

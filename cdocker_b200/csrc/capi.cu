@@ -883,7 +883,7 @@ int cdk_ctx_destroy(cdk_ctx* c) {
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
   if (c->stream) cudaStreamDestroy(c->stream);
-  cluster_release();
+  cluster_release(c->dev);
   delete c;
   return CDK_OK;
 }

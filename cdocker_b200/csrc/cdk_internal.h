@@ -272,8 +272,9 @@ void hankel_b_layout(const HankelPlan& p, WaveArgs& a);
 // the stage plan of every 128-rotation tile of a wave into the tile's first RotRec
 cudaError_t launch_tile_plan(const WaveArgs& a, int jc, cudaStream_t s);
 
-// frees the device memory and streams that the conformer clustering keeps between calls
-void cluster_release();
+// frees the device memory and streams that the conformer clustering keeps between calls on a device (-1:
+// on all); returns how many workspaces
+int cluster_release(int dev);
 
 // Digit-reversed position of natural frequency k for the radix plan of length n.
 int fft_position(int n, int k);

@@ -276,8 +276,8 @@ std::vector<int> selected_atoms(int nAtom, const unsigned char* mask) {
 // Stream and device memory of a call. An allocation, its free and a stream cost 0.8 ms of a
 // 1,000-conformer call whose kernels take 0.12 ms (and an allocation up to 12 ms on a machine in use),
 // so a few are kept between calls: at most CL_IDLE of at most CL_KEEP bytes each, one call at a time
-// on each, given back to the device by cluster_release (cdk_ctx_destroy). The list itself is never
-// destroyed: no CUDA call runs while the process exits.
+// on each, given back to the device with its contexts (cdk_ctx_destroy) or on request
+// (cdk_cluster_release). The list itself is never destroyed: no CUDA call runs while the process exits.
 constexpr size_t CL_KEEP = (size_t)32 << 20;
 constexpr size_t CL_IDLE = 2;
 
@@ -449,12 +449,27 @@ int check_inputs(int nConf, int nAtom, const double* coor, const unsigned char* 
 
 }  // namespace
 
-void cluster_release() {
-  ClusterIdle& idle = cluster_idle();
-  std::lock_guard<std::mutex> lk(idle.mu);
-  for (ClusterSpace& sp : idle.spaces)
-    if (sp.alive()) sp.drop();
-  idle.spaces.clear();
+int cluster_release(int dev) {
+  std::vector<ClusterSpace> gone;
+  {
+    ClusterIdle& idle = cluster_idle();
+    std::lock_guard<std::mutex> lk(idle.mu);
+    for (size_t i = 0; i < idle.spaces.size();) {
+      if (dev >= 0 && idle.spaces[i].dev != dev) {
+        ++i;
+        continue;
+      }
+      gone.push_back(idle.spaces[i]);
+      idle.spaces.erase(idle.spaces.begin() + i);
+    }
+  }
+  int freed = 0;
+  for (ClusterSpace& sp : gone)
+    if (sp.alive()) {
+      sp.drop();
+      ++freed;
+    }
+  return freed;
 }
 
 }  // namespace cdk
@@ -507,6 +522,8 @@ extern "C" int cdk_cluster_conformers(int nConf, int nAtom, const double* coor,
   *nCenters = count;
   return CDK_OK;
 }
+
+extern "C" int cdk_cluster_release(void) { return cluster_release(-1); }
 
 extern "C" int cdk_pair_rmsd(int nConf, int nAtom, const double* coor,
                              const unsigned char* atomMask, double* out) {

@@ -214,6 +214,11 @@ int cdk_cluster_conformers(int nConf, int nAtom, const double* coor, const doubl
 int cdk_pair_rmsd(int nConf, int nAtom, const double* coor, const unsigned char* atomMask,
                   double* out);
 
+/* The two calls above keep device memory between calls: at most two workspaces of at most 32 MB each.
+ * cdk_ctx_destroy gives back its device's; this call gives back every device's (a process that makes no
+ * context) and returns how many there were. */
+int cdk_cluster_release(void);
+
 /* ReadGrids (src/ReadGrids.cpp:6-68): header ints [numGrids, x, y, z], floats
  * [midx, midy, midz, xlen, ylen, zlen, spacing, restraint_k]; radii (numGrids-1) and values
  * (numGrids*x*y*z) are written when the capacities suffice. Pass NULL buffers to size first. */

@@ -316,13 +316,6 @@ int run_waves(cdk_ctx* c, const float* d_coor, const AtomParam* d_params, const 
   std::vector<float> osc(K);
   for (int k = 0; k < K; ++k) osc[k] = 1.f / c->lscale[k];
   const bool rows = hankel || streamed;  // the plane kernel writes split / FP16 ligand rows
-  // split-BF16 ligands that the direct plane kernel does not take (above 128 atoms): FP32 planes, rows of
-  // them and the Hankel x pass. Measured at 64^3, 100 atoms, 1,000 rotations: planes 2.0, rows 1.15,
-  // x pass 1.07 ms against 4.1 ms for the x pass that builds its operands from the planes itself
-  // (n = 64, still run on request); the direct kernel's rows take 1.0 ms in all
-  const bool convert = tc && !f16form && !rows && variant != 1 && variant != 2 &&
-                       hankel_plan(n, K, Lb, false, c->opts.reserved[5] & 3, &hp, 0, (c->opts.reserved[5] >> 2) & 7);
-  const bool hankel_x = hankel || convert;
   if (tc && f16form && !rows) {
     set_error("the split-FP16 form runs on the tensor-core x pass with ligand rows only (ligands "
               "of at most 96 atoms, a ligand box of at most 32 planes, K x n small enough for the "
@@ -331,15 +324,15 @@ int run_waves(cdk_ctx* c, const float* d_coor, const AtomParam* d_params, const 
   }
   const bool f16 = f16form && rows;
   // the Hankel x pass loads tiled ligand rows by tensor copies, or untiled rows by per-thread copies
-  const bool tiled = hankel_x && hankel_tiled(c->opts.reserved[5]);
-  const size_t lop_per = rows || convert ? stream_lop_bytes_per_rotation(n, K, f16) : 0;
+  const bool tiled = hankel && hankel_tiled(c->opts.reserved[5]);
+  const size_t lop_per = rows ? stream_lop_bytes_per_rotation(n, K, f16) : 0;
   int wave = c->opts.wave_rotations;
   if (wave <= 0) {
     // keep A + B of one wave near 16 GiB at n <= 64 (under a tenth of the B200's HBM): at 64^3,
     // waves of ~4,900 rotations instead of ~1,800 make the split-FP16 search 2-4 % faster (fewer
     // kernel tails per rotation; measured up to 8,192); 32 GiB at n >= 96, where a rotation's
     // rows and window planes take 10-30 MB
-    const double per = (double)lop_per + (rows ? 0.0 : (double)K * Lb * ncol * 8) + (double)n * ncol * 8;
+    const double per = (rows ? (double)lop_per : (double)K * Lb * ncol * 8) + (double)n * ncol * 8;
     const double target = (n <= 64 ? 16.0 : 32.0) * (1ull << 30);
     wave = (int)std::min<double>(8192.0, std::max(64.0, target / per));
   }
@@ -358,10 +351,9 @@ int run_waves(cdk_ctx* c, const float* d_coor, const AtomParam* d_params, const 
   const size_t b_A = align_up(rows ? lop_wave_bytes(wave, tiled, lop_per)
                                    : (size_t)wave * K * Lb * ncol * sizeof(float2));
   const size_t b_B = align_up(b_rotations(wave) * n * ncol * sizeof(float2));
-  const size_t b_lop = convert ? align_up(lop_wave_bytes(wave, tiled, lop_per)) : 0;  // beside the planes
-  if (!grow(c->wave, b_rotxyz + b_rec + b_keys + b_A + b_B + b_keys2 + b_lop)) {
+  if (!grow(c->wave, b_rotxyz + b_rec + b_keys + b_A + b_B + b_keys2)) {
     set_error("cudaMalloc of the wave scratch failed (" +
-              std::to_string((b_rotxyz + b_rec + b_keys + b_A + b_B + b_keys2 + b_lop) >> 20) + " MiB)");
+              std::to_string((b_rotxyz + b_rec + b_keys + b_A + b_B + b_keys2) >> 20) + " MiB)");
     return CDK_ERR_NOMEM;
   }
   char* base = static_cast<char*>(c->wave.base);
@@ -379,9 +371,7 @@ int run_waves(cdk_ctx* c, const float* d_coor, const AtomParam* d_params, const 
   a.rec = reinterpret_cast<RotRec*>(base + b_rotxyz);
   a.keys = reinterpret_cast<unsigned long long*>(base + b_rotxyz + b_rec);
   a.A = rows ? nullptr : reinterpret_cast<float2*>(base + b_rotxyz + b_rec + b_keys);
-  a.lop = rows      ? reinterpret_cast<unsigned char*>(base + b_rotxyz + b_rec + b_keys)
-          : convert ? reinterpret_cast<unsigned char*>(base + b_rotxyz + b_rec + b_keys + b_A + b_B + b_keys2)
-                    : nullptr;
+  a.lop = rows ? reinterpret_cast<unsigned char*>(base + b_rotxyz + b_rec + b_keys) : nullptr;
   a.lop_tiled = tiled ? 1 : 0;
   a.B = reinterpret_cast<float2*>(base + b_rotxyz + b_rec + b_keys + b_A);
   a.keys2 = tiebreak ? reinterpret_cast<unsigned long long*>(base + b_rotxyz + b_rec + b_keys + b_A + b_B) : nullptr;
@@ -395,7 +385,7 @@ int run_waves(cdk_ctx* c, const float* d_coor, const AtomParam* d_params, const 
   for (int k = 0; k < KMAX; ++k) a.lscale[k] = c->lscale[k];
   a.range_err = reinterpret_cast<int*>(c->d_misc + 4);
   // the shared-memory streamed x pass writes B in plane groups (whole sectors per store)
-  a.bgroup = rows || convert ? stream_bgroup() : 1;
+  a.bgroup = rows ? stream_bgroup() : 1;
   a.col_tile = c->opts.col_tile > 0 ? c->opts.col_tile : kXpassCols;
   a.kyof = (c->opts.reserved[1] & 1) ? nullptr : c->d_kyof;  // reserved[1] bit 0: FFT planes
   // bit 1: block-stage yz kernel at every n; bit 2: octet yz kernel at every n
@@ -405,7 +395,7 @@ int run_waves(cdk_ctx* c, const float* d_coor, const AtomParam* d_params, const 
     if (c->tuned_col_tile) a.col_tile = c->tuned_col_tile;
     a.chunk = c->tuned_chunk;
   }
-  if (tc && !rows && !convert && xpass_tc_smem_bytes(n, K, Lb) > 227 * 1024) {
+  if (tc && !rows && xpass_tc_smem_bytes(n, K, Lb) > 227 * 1024) {
     set_error("ligand box too large for the tensor-core x pass at this grid size and K");
     return CDK_ERR_UNSUPPORTED;
   }
@@ -415,7 +405,7 @@ int run_waves(cdk_ctx* c, const float* d_coor, const AtomParam* d_params, const 
   }
   CDK_CUDA(cudaMemsetAsync(c->d_misc + 2, 0, 3 * sizeof(unsigned int), s));
   CDK_CUDA(cudaMemsetAsync(c->d_work, 0, 8 * sizeof(unsigned long long), s));
-  const bool umma = tc && !rows && !convert && variant != 1 && umma_supported(n, Lb);
+  const bool umma = tc && !rows && variant != 1 && umma_supported(n, Lb);
   a.work = c->d_work;
   const bool prof = c->opts.reserved[0] != 0;
   const long nwaves = (nRot + wave - 1) / wave;
@@ -440,7 +430,7 @@ int run_waves(cdk_ctx* c, const float* d_coor, const AtomParam* d_params, const 
   CDK_CUDA(cudaStreamIsCapturing(s, &cap_state));
   const unsigned int evflags = cap_state == cudaStreamCaptureStatusActive ? cudaEventRecordExternal
                                                                           : cudaEventRecordDefault;
-  if (c->opts.reserved[2] && c->tuned_Lb != Lb && !rows && !convert) {
+  if (c->opts.reserved[2] && c->tuned_Lb != Lb && !rows) {
     int rc = autotune_xpass(c, a, d_rots, nRot, wave, tc, s);
     if (rc) return rc;
     a.col_tile = c->tuned_col_tile ? c->tuned_col_tile : a.col_tile;
@@ -451,7 +441,7 @@ int run_waves(cdk_ctx* c, const float* d_coor, const AtomParam* d_params, const 
   // K-steps per 128-rotation tile; reserved[4] = 1 keeps the given order)
   const RotDesc* order = d_rots;
   const int jc = (Lb + 7) / 8;
-  if ((rows || convert) && c->opts.reserved[4] == 0 && nRot > 128 && jc > 1) {
+  if (rows && c->opts.reserved[4] == 0 && nRot > 128 && jc > 1) {
     const size_t gb = group_rotations_bytes(nRot);
     if (!grow(c->group, gb)) {
       set_error("cudaMalloc of the rotation-grouping scratch failed (" + std::to_string(gb >> 20) + " MiB)");
@@ -469,7 +459,7 @@ int run_waves(cdk_ctx* c, const float* d_coor, const AtomParam* d_params, const 
   }
   if (hankel && c->tuned_hx_Lb == Lb && c->tuned_hx_cols > 0)
     hankel_plan(n, K, Lb, f16form, c->tuned_hx_cols, &hp, c->tuned_hx_nb, c->tuned_hx_ks);
-  if (hankel_x) hankel_b_layout(hp, a);
+  if (hankel) hankel_b_layout(hp, a);
   else if (!tc && a.yz_block_stages == 0) a.bpairs = 2;  // the FP32 x pass writes plane pairs
   if (c->opts.reserved[2]) c->tuned_any_Lb = Lb;
   for (long r0 = 0; r0 < nRot; r0 += wave) {
@@ -480,9 +470,9 @@ int run_waves(cdk_ctx* c, const float* d_coor, const AtomParam* d_params, const 
     if (prof) CDK_CUDA(cudaEventRecordWithFlags(ev[0], s, evflags));
     CDK_CUDA(launch_prep(a, s));
     if (prof) CDK_CUDA(cudaEventRecordWithFlags(ev[1], s, evflags));
-    CDK_CUDA(convert ? launch_rows_from_planes(a, s) : launch_spread_yz(a, s));
+    CDK_CUDA(launch_spread_yz(a, s));
     if (prof) CDK_CUDA(cudaEventRecordWithFlags(ev[2], s, evflags));
-    if (hankel_x) CDK_CUDA(launch_xpass_hankel(a, c->d_ptilde, osc.data(), hp, s));
+    if (hankel) CDK_CUDA(launch_xpass_hankel(a, c->d_ptilde, osc.data(), hp, s));
     else if (streamed) CDK_CUDA(launch_xpass_stream(a, c->d_top, s));
     else if (umma) CDK_CUDA(launch_xpass_umma(a, c->d_ptilde, s));
     else if (tc) CDK_CUDA(launch_xpass_tc(a, c->d_ptilde, s));
@@ -495,7 +485,7 @@ int run_waves(cdk_ctx* c, const float* d_coor, const AtomParam* d_params, const 
       CDK_CUDA(launch_finalize_topk(a, c->d_grids, topk, static_cast<TopPose*>(c->topk.base) + (size_t)waves * topk, s));
     else CDK_CUDA(launch_finalize(a, s));
     if (prof) CDK_CUDA(cudaEventRecordWithFlags(ev[5], s, evflags));
-    launches += kLaunchesPerWave + (rows ? 1 : convert ? 2 : 0) + (tiebreak ? 1 : 0);  // + k_tile_plan (and the rows of planes)
+    launches += kLaunchesPerWave + (rows ? 1 : 0) + (tiebreak ? 1 : 0);  // + k_tile_plan
     ++waves;
   }
   c->kev_used = prof ? (int)waves : 0;
@@ -505,9 +495,9 @@ int run_waves(cdk_ctx* c, const float* d_coor, const AtomParam* d_params, const 
   c->stats[2] = (double)nRot;
   c->stats[4] = (double)Lb;
   c->stats[5] = (double)wave;
-  c->stats[13] = hankel_x ? (double)hp.cols : streamed ? 4.0 : (double)a.col_tile;
-  c->stats[14] = rows || convert || umma ? 128.0 : tc ? (double)(a.chunk > 0 ? a.chunk : 64) : (double)xpass_rotations_per_cta(a);
-  c->stats[16] = hankel && direct_planes(probe) ? (f16 ? 7.0 : 6.0) : streamed ? (f16 ? 5.0 : 3.0) : hankel_x || umma ? 2.0 : tc ? 1.0 : 0.0;
+  c->stats[13] = hankel ? (double)hp.cols : streamed ? 4.0 : (double)a.col_tile;
+  c->stats[14] = rows || umma ? 128.0 : tc ? (double)(a.chunk > 0 ? a.chunk : 64) : (double)xpass_rotations_per_cta(a);
+  c->stats[16] = hankel && direct_planes(probe) ? (f16 ? 7.0 : 6.0) : streamed ? (f16 ? 5.0 : 3.0) : hankel || umma ? 2.0 : tc ? 1.0 : 0.0;
   c->stats[15] = (double)(c->gkey_seen);
   return CDK_OK;
 }

@@ -191,8 +191,6 @@ cudaError_t launch_group_rotations(const RotDesc* rots, const ConfDesc* confs, c
                                    const AtomParam* params, long nrot, int max_atoms, int K, float h,
                                    int jc, void* scratch, RotDesc** sorted, cudaStream_t s);
 cudaError_t launch_spread_yz(const WaveArgs& a, cudaStream_t s);
-// FP32 planes into a.A, then split-BF16 ligand rows of them into a.lop (both layouts)
-cudaError_t launch_rows_from_planes(const WaveArgs& a, cudaStream_t s);
 cudaError_t launch_xpass(const WaveArgs& a, cudaStream_t s);
 cudaError_t launch_yz_inv_argmin(const WaveArgs& a, cudaStream_t s);
 // the inverse (y,z) pass over paired planes (WaveArgs.bpairs), and the key pairs per rotation it

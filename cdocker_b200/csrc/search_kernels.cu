@@ -405,48 +405,6 @@ __device__ __forceinline__ void tile_plan_range(const WaveArgs& a, int r, int k,
     }
 }
 
-// Split-BF16 ligand rows from FP32 planes (A), for ligands that the direct plane kernel does not
-// take: per (rotation, channel) the chunks of the tile's stage plan (tiled rows; zeros where the
-// channel has no plane) or its own chunks. Bound: DRAM (8 bytes read and, with the hi and lo parts,
-// 8 written per plane and column); two columns per thread, so that loads and stores are 16 and 128
-// bytes.
-template <int N>
-__global__ void __launch_bounds__(256) k_rows_from_planes(const __grid_constant__ WaveArgs a) {
-  constexpr int NCOL = N * (N / 2 + 1);
-  const int r = blockIdx.x, k = blockIdx.y;
-  const RotRec* rec = a.rec + r;
-  if (!rec->valid) return;
-  const int xlo = rec->xlo[k], xhi = rec->xhi[k];
-  int lo = 1, hi = 0;
-  if (xlo <= xhi) lo = xlo >> 3, hi = xhi >> 3;
-  if (a.lop_tiled) tile_plan_range(a, r, k, lo, hi);
-  const float2* src = a.A + ((size_t)r * a.K + k) * a.Lb * NCOL;
-  for (int i = threadIdx.x; i < (hi - lo + 1) * (NCOL / 2); i += 256) {
-    const int q = lo + i / (NCOL / 2), c = i % (NCOL / 2) * 2;
-    uint32_t h[2][16];
-#pragma unroll
-    for (int d = 0; d < 8; d += 2) {
-      float4 v[2];
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int x = 8 * q + d + e;
-        v[e] = x >= xlo && x <= xhi ? *reinterpret_cast<const float4*>(src + (size_t)x * NCOL + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-      split_bf16x2(v[0].x, v[1].x, h[0][d / 2], h[0][8 + d / 2]);
-      split_bf16x2(v[0].y, v[1].y, h[0][4 + d / 2], h[0][12 + d / 2]);
-      split_bf16x2(v[0].z, v[1].z, h[1][d / 2], h[1][8 + d / 2]);
-      split_bf16x2(v[0].w, v[1].w, h[1][4 + d / 2], h[1][12 + d / 2]);
-    }
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      uint4 rows[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) rows[j] = make_uint4(h[u][4 * j], h[u][4 * j + 1], h[u][4 * j + 2], h[u][4 * j + 3]);
-      plane_rows_write<N, kRowsBf16>(a, r, k, q, c + u, rows);
-    }
-  }
-}
-
 // Largest ligand of the direct plane kernel: 96 atoms; split-BF16 rows up to 128 (FP32 planes stay
 // with FillLigandGrid's rounding above 96, and the split-FP16 form refuses larger ligands)
 constexpr int direct_max_atoms(int rows) { return rows == kRowsBf16 ? 128 : 96; }
@@ -1627,21 +1585,6 @@ cudaError_t launch_spread_yz(const WaveArgs& a, cudaStream_t s) {
     if (e != cudaSuccess) return e;
   }
   CDK_DISPATCH_N(a.n, launch_spread_yz_t, a, s);
-}
-template <int N>
-static cudaError_t launch_rows_t(const WaveArgs& a, cudaStream_t s) {
-  k_rows_from_planes<N><<<dim3(a.nrot, a.K), 256, 0, s>>>(a);
-  return cudaGetLastError();
-}
-cudaError_t launch_rows_from_planes(const WaveArgs& a, cudaStream_t s) {
-  if (!a.A || !a.lop || a.f16 || (reinterpret_cast<uintptr_t>(a.lop) & 127)) return cudaErrorInvalidValue;
-  WaveArgs p = a;  // the planes first, then the rows
-  p.lop = nullptr;
-  p.lop_tiled = 0;
-  cudaError_t e = launch_spread_yz(p, s);
-  if (e == cudaSuccess && a.lop_tiled) e = launch_tile_plan(a, (a.Lb + 7) / 8, s);
-  if (e != cudaSuccess) return e;
-  CDK_DISPATCH_N(a.n, launch_rows_t, a, s);
 }
 bool direct_planes(const WaveArgs& a) {
   const int cap = a.atom_cap > 0 ? a.atom_cap : a.max_atoms;

@@ -298,8 +298,7 @@ int run_waves(cdk_ctx* c, const float* d_coor, const AtomParam* d_params, const 
   const bool can_stream = tc && stream_supported(n, Lb) && direct_planes(probe);
   const bool streamed = can_stream && use_stream_tiles(variant);
   HankelPlan hp{};
-  const bool hankel = tc && !streamed && (variant == 0 || variant == 4) &&
-                      (f16form ? direct_planes(probe) : direct_rows_bf16(probe)) &&
+  const bool hankel = tc && !streamed && (variant == 0 || variant == 4) && direct_planes(probe) &&
                       hankel_plan(n, K, Lb, f16form, c->opts.reserved[5] & 3, &hp, 0, (c->opts.reserved[5] >> 2) & 7);
   if (streamed && !c->d_top) {
     const size_t tb = stream_top_bytes(n, K);
@@ -497,7 +496,7 @@ int run_waves(cdk_ctx* c, const float* d_coor, const AtomParam* d_params, const 
   c->stats[5] = (double)wave;
   c->stats[13] = hankel ? (double)hp.cols : streamed ? 4.0 : (double)a.col_tile;
   c->stats[14] = rows || umma ? 128.0 : tc ? (double)(a.chunk > 0 ? a.chunk : 64) : (double)xpass_rotations_per_cta(a);
-  c->stats[16] = hankel && direct_planes(probe) ? (f16 ? 7.0 : 6.0) : streamed ? (f16 ? 5.0 : 3.0) : hankel || umma ? 2.0 : tc ? 1.0 : 0.0;
+  c->stats[16] = hankel ? (f16 ? 7.0 : 6.0) : streamed ? (f16 ? 5.0 : 3.0) : umma ? 2.0 : tc ? 1.0 : 0.0;
   c->stats[15] = (double)(c->gkey_seen);
   return CDK_OK;
 }

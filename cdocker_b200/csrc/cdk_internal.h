@@ -102,8 +102,7 @@ struct WaveArgs {
   int chunk;                 // rotations per CTA in the x pass (0 = default)
   int* fault;                // set when a bounded device wait gave up
   const int* kyof;           // [n] natural frequency at each digit-reversed position; when set
-                             // (and ligands have <= 96 atoms, split-BF16 rows 128) planes are
-                             // evaluated directly
+                             // (and ligands have <= 96 atoms) planes are evaluated directly
   int f16;                   // split-FP16 form: the plane kernel writes FP16 rows (8 per rotation
                              // and channel: [chunk][re, im]) of the planes times lscale[k]
   float lscale[KMAX];        // split-FP16 form: 2^sigma_k per channel (a power of two, exact)
@@ -242,10 +241,8 @@ int stream_bgroup();
 cudaError_t launch_top_build(int n, int K, const float2* pt, void* top, const float* f16_scale,
                              cudaStream_t s);
 cudaError_t launch_xpass_stream(const WaveArgs& a, const void* top, cudaStream_t s);
-// true when launch_spread_yz takes the direct plane path (the only one that can write lop); with
-// split-BF16 rows it takes larger ligands
+// true when launch_spread_yz takes the direct plane path (the only one that can write lop)
 bool direct_planes(const WaveArgs& a);
-bool direct_rows_bf16(const WaveArgs& a);
 
 // tcgen05 x pass with the Hankel operator resident in shared memory (any n, ligand box <= 32
 // planes): its shape for (n, K, box, form) and its launch (k_tile_plan, then the x pass)

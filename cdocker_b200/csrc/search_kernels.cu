@@ -405,9 +405,9 @@ __device__ __forceinline__ void tile_plan_range(const WaveArgs& a, int r, int k,
     }
 }
 
-// Largest ligand of the direct plane kernel: 96 atoms; split-BF16 rows up to 128 (FP32 planes stay
-// with FillLigandGrid's rounding above 96, and the split-FP16 form refuses larger ligands)
-constexpr int direct_max_atoms(int rows) { return rows == kRowsBf16 ? 128 : 96; }
+// Largest ligand of the direct plane kernel (larger ones keep FillLigandGrid's 64-bit weights, in the FFT
+// planes)
+constexpr int kDirectMaxAtoms = 96;
 
 // Shape of the direct plane kernel: threads per CTA and CTAs per SM asked for (registers), shared
 // memory for ligands of at most cap atoms
@@ -455,7 +455,7 @@ __global__ void __launch_bounds__(DirectShape<N, ROWS>::T, DirectShape<N, ROWS>:
   float2* Fz = reinterpret_cast<float2*>(Fy + (size_t)cap * NY * 2);  // [cap][NZH]
   float2* tw = Fz + (size_t)cap * NZH;                             // [N]
   float2* s_rr = tw + N;                                           // [cap] y and z ratios
-  constexpr int kDirectWords = direct_max_atoms(ROWS) / 32;
+  constexpr int kDirectWords = kDirectMaxAtoms / 32;
   __shared__ uint32_t s_plane[N][kDirectWords];   // atoms with a cell on the plane (bit j)
   __shared__ uint32_t s_chan[KMAX][kDirectWords];  // atoms of the channel
   __shared__ uint32_t s_run[KMAX][N];             // list entries of (channel, plane): first | count << 16
@@ -1336,21 +1336,21 @@ constexpr size_t plane_smem() {
 template <int N>
 cudaError_t launch_spread_yz_t(const WaveArgs& a, cudaStream_t s) {
   const int cap = a.atom_cap > 0 ? a.atom_cap : a.max_atoms;
-  if (a.kyof && cap <= direct_max_atoms(!a.lop ? kRowsNone : a.f16 ? kRowsF16 : kRowsBf16)) {
-    auto launch = [&](auto kern, auto shape, int rows) {
+  if (a.kyof && cap <= kDirectMaxAtoms) {
+    auto launch = [&](auto kern, auto shape) {
       // room for the largest ligand whatever this one's atoms: the attribute is the process's, and another
       // thread's smaller ligand, set between this call and the launch, would refuse it
       const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)shape.smem(direct_max_atoms(rows)));
+                                                 (int)shape.smem(kDirectMaxAtoms));
       if (e != cudaSuccess) return e;
       // parts of a rotation's items: enough CTAs for small waves (each part repeats the tables)
       const int parts = std::max(1, std::min(a.K, (148 * 6 + a.nrot - 1) / a.nrot));
       kern<<<dim3(parts, a.nrot), shape.T, shape.smem(cap), s>>>(a, a.kyof, cap);
       return cudaGetLastError();
     };
-    if (!a.lop) return launch(k_spread_yz_direct<N, kRowsNone>, DirectShape<N, kRowsNone>{}, kRowsNone);
-    if (a.f16) return launch(k_spread_yz_direct<N, kRowsF16>, DirectShape<N, kRowsF16>{}, kRowsF16);
-    return launch(k_spread_yz_direct<N, kRowsBf16>, DirectShape<N, kRowsBf16>{}, kRowsBf16);
+    if (!a.lop) return launch(k_spread_yz_direct<N, kRowsNone>, DirectShape<N, kRowsNone>{});
+    if (a.f16) return launch(k_spread_yz_direct<N, kRowsF16>, DirectShape<N, kRowsF16>{});
+    return launch(k_spread_yz_direct<N, kRowsBf16>, DirectShape<N, kRowsBf16>{});
   }
   if (a.lop) return cudaErrorInvalidValue;  // the FFT plane path writes A only
   const size_t sm = plane_smem<N>();
@@ -1580,7 +1580,7 @@ cudaError_t launch_prep(const WaveArgs& a, cudaStream_t s) {
 cudaError_t launch_spread_yz(const WaveArgs& a, cudaStream_t s) {
   if (a.lop_tiled) {
     // the tiled rows zero-fill by the tiles' stage plans: k_tile_plan first
-    if (!a.lop || !(a.f16 ? direct_planes(a) : direct_rows_bf16(a)) || (reinterpret_cast<uintptr_t>(a.lop) & 127)) return cudaErrorInvalidValue;
+    if (!a.lop || !direct_planes(a) || (reinterpret_cast<uintptr_t>(a.lop) & 127)) return cudaErrorInvalidValue;
     cudaError_t e = launch_tile_plan(a, (a.Lb + 7) / 8, s);
     if (e != cudaSuccess) return e;
   }
@@ -1588,11 +1588,7 @@ cudaError_t launch_spread_yz(const WaveArgs& a, cudaStream_t s) {
 }
 bool direct_planes(const WaveArgs& a) {
   const int cap = a.atom_cap > 0 ? a.atom_cap : a.max_atoms;
-  return a.kyof != nullptr && cap <= direct_max_atoms(kRowsNone);
-}
-bool direct_rows_bf16(const WaveArgs& a) {
-  const int cap = a.atom_cap > 0 ? a.atom_cap : a.max_atoms;
-  return a.kyof != nullptr && cap <= direct_max_atoms(kRowsBf16);
+  return a.kyof != nullptr && cap <= kDirectMaxAtoms;
 }
 cudaError_t launch_yz_inv_argmin(const WaveArgs& a, cudaStream_t s) {
   if (a.bpairs) return launch_yz_pairs(a, s);

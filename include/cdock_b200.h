@@ -62,9 +62,8 @@ typedef struct cdk_opts {
                           the x pass writes plane pairs or quads); [2] = 1: autotune the x pass on the first wave
                           of each new ligand box; [3] precision-form x pass: 0 = automatic
                           (ligands <= 96 atoms, box <= 32 planes: tcgen05 with the Hankel
-                          operator resident in shared memory, split-BF16 up to 128 atoms; else,
-                          split-BF16 only, the next one at n = 64 and box <= 32, mma.sync
-                          otherwise); 1 = mma.sync;
+                          operator resident in shared memory; else, split-BF16 only: n = 64 and
+                          box <= 32 planes the next but one, mma.sync otherwise); 1 = mma.sync;
                           2 = tcgen05 with operands built inside the kernel (n = 64);
                           3 = streamed operator tiles (n = 64); 4 = the Hankel kernel;
                           [4] = 1: keep the rotations in the given order in the streamed
@@ -301,9 +300,7 @@ int cdk_server_destroy(cdk_server* s);
  * kind (prep, spread_yz, xpass, yz_inv_argmin with the near-tie break, finalize with the top poses) when the context was created with
  * opts.reserved[0] = 1 (events around every launch), else 0; [13] x-pass column tile (FP32 form: opts.col_tile, 8 when 0),
  * [14] x-pass rotations per CTA, [15] graph state (0 off, 1 shape seen, 2 replaying),
- * [16] x-pass kind (0 FP32 radix, 1 mma.sync, 2 tcgen05 for split-BF16 ligands above 96 atoms:
- * the resident Hankel operator (up to 128 atoms), or at n = 64 operands built from the planes inside
- * the x pass (also on request),
+ * [16] x-pass kind (0 FP32 radix, 1 mma.sync, 2 tcgen05 with in-kernel operand builds,
  * 3 tcgen05 with streamed operator tiles (64^3), 5 the same in the split-FP16 form,
  * 6 tcgen05 with the resident Hankel operator, 7 the same in the split-FP16 form),
  * [17] tensor-core K-steps the x pass issued per spectral column (one step = the MMAs of one

@@ -1,5 +1,5 @@
-"""Split-BF16 searches off the direct plane path (ligands above 128 atoms, planes by the FFT): the same bits
-and the same kind as the x pass that such ligands always had, in-kernel operand builds at 64^3 and mma.sync
+"""Split-BF16 searches off the direct plane path (ligands above 96 atoms, planes by the FFT): the same bits and
+the same kind as the x pass that such ligands always had, in-kernel operand builds at 64^3 and mma.sync
 at the other grids, whatever the number of rotations."""
 import numpy as np
 import pytest
@@ -24,7 +24,8 @@ def search(n, K, atoms, rots, length=9.0, **kw):
 
 
 @pytest.mark.parametrize("n,K,atoms,rots,kw", [
-    (32, 4, 129, 3, {}), (64, 9, 129, 200, {}), (64, 3, 250, 1, {}), (96, 4, 160, 5, {}), (128, 3, 129, 2, {}),
+    (32, 9, 97, 40, {}), (64, 9, 100, 300, {}), (64, 2, 97, 1, {}), (64, 9, 128, 130, {}), (96, 9, 110, 3, {}),
+    (128, 4, 97, 2, {}), (64, 9, 110, 40, {"tc_hankel": True}), (32, 4, 129, 3, {}), (64, 9, 129, 200, {}), (64, 3, 250, 1, {}), (96, 4, 160, 5, {}), (128, 3, 129, 2, {}),
     (32, 4, 40, 150, {"fft_planes": True}), (64, 9, 40, 30, {"fft_planes": True})])
 def test_same_x_pass_as_asked_for(n, K, atoms, rots, kw):
     other = {"tc_build": True} if n == 64 else {"tc_mma_sync": True}

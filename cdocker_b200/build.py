@@ -27,7 +27,7 @@ NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xptxas"
 CXX_FLAGS = ["-O2", "-std=c++14", "-fPIC", "-ffp-contract=off", "-Wno-deprecated-declarations",
              "-pthread"]
 
-CU_SOURCES = ["search_kernels.cu", "fp32_xpass.cu", "yz_pairs.cu", "compat_kernels.cu", "capi.cu", "noalloc.cu", "server.cu", "tc_xpass.cu", "umma_xpass.cu",
+CU_SOURCES = ["search_kernels.cu", "fp32_xpass.cu", "block_xpass.cu", "yz_pairs.cu", "compat_kernels.cu", "capi.cu", "noalloc.cu", "server.cu", "tc_xpass.cu", "umma_xpass.cu",
               "cluster.cu", "stream_xpass.cu", "hankel_xpass.cu", "receptor_grids.cu"]
 CPP_SOURCES = ["host/reference_api.cpp"]
 

@@ -459,11 +459,11 @@ int run_waves(cdk_ctx* c, const float* d_coor, const AtomParam* d_params, const 
   if (hankel && c->tuned_hx_Lb == Lb && c->tuned_hx_cols > 0)
     hankel_plan(n, K, Lb, f16form, c->tuned_hx_cols, &hp, c->tuned_hx_nb, c->tuned_hx_ks);
   if (hankel) hankel_b_layout(hp, a);
-  else if (!tc && a.yz_block_stages == 0) a.bpairs = 2;  // the FP32 x pass writes plane pairs
   if (c->opts.reserved[2]) c->tuned_any_Lb = Lb;
   for (long r0 = 0; r0 < nRot; r0 += wave) {
     a.nrot = (int)std::min<long>(wave, nRot - r0);
     a.rots = order + r0;
+    if (!tc) xpass_b_layout(a);
     a.key_slots = a.bpairs ? yz_pairs_key_slots(a) : 0;
     cudaEvent_t* ev = prof ? &c->kev[(size_t)waves * (kLaunchesPerWave + 1)] : nullptr;
     if (prof) CDK_CUDA(cudaEventRecordWithFlags(ev[0], s, evflags));
@@ -494,7 +494,7 @@ int run_waves(cdk_ctx* c, const float* d_coor, const AtomParam* d_params, const 
   c->stats[2] = (double)nRot;
   c->stats[4] = (double)Lb;
   c->stats[5] = (double)wave;
-  c->stats[13] = hankel ? (double)hp.cols : streamed ? 4.0 : (double)a.col_tile;
+  c->stats[13] = hankel ? (double)hp.cols : streamed ? 4.0 : tc ? (double)a.col_tile : (double)xpass_columns_per_cta(a);
   c->stats[14] = rows || umma ? 128.0 : tc ? (double)(a.chunk > 0 ? a.chunk : 64) : (double)xpass_rotations_per_cta(a);
   c->stats[16] = hankel ? (f16 ? 7.0 : 6.0) : streamed ? (f16 ? 5.0 : 3.0) : umma ? 2.0 : tc ? 1.0 : 0.0;
   c->stats[15] = (double)(c->gkey_seen);

@@ -190,7 +190,14 @@ cudaError_t launch_group_rotations(const RotDesc* rots, const ConfDesc* confs, c
                                    const AtomParam* params, long nrot, int max_atoms, int K, float h,
                                    int jc, void* scratch, RotDesc** sorted, cudaStream_t s);
 cudaError_t launch_spread_yz(const WaveArgs& a, cudaStream_t s);
+// FP32 x pass. Its B layout (WaveArgs.bpairs) is set for the wave by xpass_b_layout: plane pairs, or the plain
+// one where the inverse kernel asked for or the x pass of such a wave (xpass_block_stages) has no pairs
 cudaError_t launch_xpass(const WaveArgs& a, cudaStream_t s);
+cudaError_t launch_xpass_block(const WaveArgs& a, cudaStream_t s);
+bool xpass_block_stages(const WaveArgs& a);
+int xpass_block_columns(int n, int K);
+constexpr int kXpassBlockRotations = 32;
+void xpass_b_layout(WaveArgs& a);
 cudaError_t launch_yz_inv_argmin(const WaveArgs& a, cudaStream_t s);
 // the inverse (y,z) pass over paired planes (WaveArgs.bpairs), and the key pairs per rotation it
 // writes (WaveArgs.key_slots)
@@ -203,12 +210,13 @@ cudaError_t launch_finalize_server(const WaveArgs& a, float* ebase, int* ibase, 
 // Dense forward transform of K receptor grids [K][n][n][n] -> phat [n][K][ncol].
 cudaError_t launch_receptor_fft(int n, int K, const float* grids, float2* scratch,
                                 float2* phat, const float2* tw, int col_tile, cudaStream_t s);
-// Column tiles opts.col_tile may name (8, or 16 at n <= 64); the FP32 x pass runs 8 columns per CTA
-// whichever is named, with the same results.
+// Column tiles opts.col_tile may name (8, or 16 at n <= 64); the FP32 x pass runs its own choice, with the
+// same results whichever is named.
 bool xpass_col_tile_ok(int n, int col_tile);
 constexpr int kXpassCols = 8;
-// rotations per CTA of the FP32 x pass for this wave
+// rotations and columns per CTA of the FP32 x pass for this wave (layout set)
 int xpass_rotations_per_cta(const WaveArgs& a);
+int xpass_columns_per_cta(const WaveArgs& a);
 // Dense FillLigandGrid on the GPU.
 cudaError_t launch_fill_dense(int nQ, int nAtom, const float* coors, const float* mincoors,
                               const AtomParam* params, int nVdwUsed, int X, int Y, int Z,

@@ -237,10 +237,10 @@ extern "C" int cdk_search_device_noalloc(cdk_ctx* ctx, int nAtom, int nConf,
   a.work = reinterpret_cast<unsigned long long*>(misc + 4);
   a.col_tile = v.col_tile_opt > 0 ? v.col_tile_opt : kXpassCols;
   a.kyof = v.kyof;
-  a.bpairs = 2;
   for (long r0 = 0; r0 < nRot; r0 += wave) {
     a.nrot = (int)std::min<long>(wave, nRot - r0);
     a.rots = rots;
+    xpass_b_layout(a);
     const long tmax = std::max<long>(a.nrot, std::max(nConf, nAtom));
     k_na_tables<<<(unsigned)((tmax + 255) / 256), 256, 0, s>>>(
         r0, a.nrot, nAtom, nConf, nQ, d_quats, d_charge, d_eps, d_slot, confs, rots, params);

@@ -413,10 +413,9 @@ void worker_loop(cdk_server* s) {
     a.f16 = (tc_wave && f16) ? 1 : 0;
     a.bgroup = tc_wave ? stream_bgroup() : 1;
     a.bcol = 0;
-    // the FP32 x pass writes plane pairs, but for the inverse kernels that keep the near-tie break's two
-    // smallest keys the plain layout: over plane pairs there is none with them
-    a.bpairs = tc_wave || a.keys2 ? 0 : 2;
-    if (tc_wave && !tile_wave) hankel_b_layout(hp, a);
+    a.bpairs = 0;
+    if (!tc_wave) xpass_b_layout(a);
+    else if (!tile_wave) hankel_b_layout(hp, a);
     a.key_slots = a.bpairs ? yz_pairs_key_slots(a) : 0;
     if (le == cudaSuccess) {
       note(launch_prep(a, s->stream));

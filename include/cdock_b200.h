@@ -51,8 +51,8 @@ typedef struct cdk_opts {
   int form;            /* CDK_FORM_* */
   int wave_rotations;  /* rotations per launch wave; 0 = pick automatically */
   int max_atoms;       /* largest ligand (atoms) this context will see; 0 = 256 */
-  int col_tile;        /* accepted for the FP32 x pass: 0, 8, or 16 (n <= 64); it runs 8 spectral
-                          columns per CTA whichever is named, with the same results */
+  int col_tile;        /* accepted for the FP32 x pass: 0, 8, or 16 (n <= 64); it runs its own choice
+                          of spectral columns per CTA whichever is named, with the same results */
   int use_graphs;      /* 1 = replay each wave through a captured CUDA graph */
   int reserved[8];     /* [0] = 1: time every kernel with events (cdk_ctx_stats [8..12]);
                           [1] bit 0: spread planes through the radix FFT instead of the direct
@@ -298,7 +298,8 @@ int cdk_server_destroy(cdk_server* s);
  * search stream), [4] planned ligand box edge, [5] rotations per wave, [6] (y,z) planes the
  * spread kernel transformed, [7] window planes the x pass wrote, [8..12] device ms per kernel
  * kind (prep, spread_yz, xpass, yz_inv_argmin with the near-tie break, finalize with the top poses) when the context was created with
- * opts.reserved[0] = 1 (events around every launch), else 0; [13] x-pass column tile (FP32 form: opts.col_tile, 8 when 0),
+ * opts.reserved[0] = 1 (events around every launch), else 0; [13] x-pass columns per CTA (of the
+ * last wave),
  * [14] x-pass rotations per CTA, [15] graph state (0 off, 1 shape seen, 2 replaying),
  * [16] x-pass kind (0 FP32 radix, 1 mma.sync, 2 tcgen05 with in-kernel operand builds,
  * 3 tcgen05 with streamed operator tiles (64^3), 5 the same in the split-FP16 form,

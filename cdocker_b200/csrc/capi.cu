@@ -164,73 +164,85 @@ namespace {
 
 bool supported_n(int n) { return n == 32 || n == 64 || n == 96 || n == 128; }
 
-// Times the x pass (the dominant kernel) on the search's first wave under each candidate
-// configuration (rotations per CTA) and keeps the fastest for this ligand box. The candidates all compute
-// the same numbers (deterministic kernels), so the timing runs leave no trace in the results.
-int autotune_xpass(cdk_ctx* c, WaveArgs a, const RotDesc* d_rots, long nRot, int wave, bool tc,
-                   cudaStream_t s) {
+// Times the FP32 or the mma.sync x pass on the search's first wave under each candidate configuration (rotations
+// per CTA) and keeps the fastest for this ligand box. The candidates all compute the same numbers (deterministic
+// kernels), so the timing runs leave no trace in the results.
+// The FP32 x pass has candidates for small waves only. From 256 rotations on its plan's own chunk stands, chosen
+// for the wave's rotation count: over 204 shapes (every n, K 2 to 16, 30 to 4,000 rotations) none of nine others
+// was faster by more than the timer's step, and a fixed one is slower (64 rotations per CTA: x pass 155 against
+// 144 ms per 1e5 rotations at 64^3). Below, callers find 16, 32 or 64 in the statistics.
+constexpr int kTunedFp32Rotations = 256;
+int autotune_xpass(cdk_ctx* c, WaveArgs a, const RotDesc* d_rots, long nRot, int wave, bool tc, cudaStream_t s) {
   a.nrot = (int)std::min<long>(wave, nRot);
   a.rots = d_rots;
-  CDK_CUDA(launch_prep(a, s));
-  CDK_CUDA(launch_spread_yz(a, s));
   struct Cand { int ct, chunk; };
   std::vector<Cand> cands;
-  if (tc && c->opts.reserved[3] != 1 && umma_supported(c->n, a.Lb)) {
-    cands.push_back({a.col_tile, 0});  // fixed 128-rotation tiles
+  if (tc ? c->opts.reserved[3] != 1 && umma_supported(c->n, a.Lb) : a.nrot >= kTunedFp32Rotations) {
+    cands.push_back({a.col_tile, 0});  // nothing to try: fixed 128-rotation tiles, the plan's own chunk
   } else if (tc) {
     for (int ch : {32, 64, 128, 256}) cands.push_back({a.col_tile, ch});
   } else {
+    xpass_b_layout(a);  // the stores that the search makes
     for (int ch : {16, 32, 64}) cands.push_back({a.col_tile, ch});
   }
-  cudaEvent_t e0, e1;
-  CDK_CUDA(cudaEventCreate(&e0));
-  CDK_CUDA(cudaEventCreate(&e1));
-  double best = 1e30;
   Cand pick = cands[0];
-  int i = 0;
-  for (const Cand& cd : cands) {
-    WaveArgs t = a;
-    t.col_tile = cd.ct;
-    t.chunk = cd.chunk;
-    float ms = 0.f, total = 0.f;
-    for (int rep = 0; rep < 2; ++rep) {
-      CDK_CUDA(cudaEventRecord(e0, s));
-      if (tc && c->opts.reserved[3] != 1 && umma_supported(c->n, a.Lb))
-        CDK_CUDA(launch_xpass_umma(t, c->d_ptilde, s));
-      else if (tc) CDK_CUDA(launch_xpass_tc(t, c->d_ptilde, s));
-      else CDK_CUDA(launch_xpass(t, s));
-      CDK_CUDA(cudaEventRecord(e1, s));
-      CDK_CUDA(cudaEventSynchronize(e1));
-      CDK_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-      if (rep == 1) total = ms;  // second run: warm caches
+  if (cands.size() > 1) {
+    CDK_CUDA(launch_prep(a, s));
+    CDK_CUDA(launch_spread_yz(a, s));
+    cudaEvent_t e0, e1;
+    CDK_CUDA(cudaEventCreate(&e0));
+    CDK_CUDA(cudaEventCreate(&e1));
+    double best = 1e30;
+    int i = 0;
+    for (const Cand& cd : cands) {
+      WaveArgs t = a;
+      t.col_tile = cd.ct;
+      t.chunk = cd.chunk;
+      float ms = 0.f, total = 0.f;
+      for (int rep = 0; rep < 2; ++rep) {
+        CDK_CUDA(cudaEventRecord(e0, s));
+        if (tc) CDK_CUDA(launch_xpass_tc(t, c->d_ptilde, s));
+        else CDK_CUDA(launch_xpass(t, s));
+        CDK_CUDA(cudaEventRecord(e1, s));
+        CDK_CUDA(cudaEventSynchronize(e1));
+        CDK_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+        if (rep == 1) total = ms;  // second run: warm caches
+      }
+      if (i < 8) c->tune_ms[i] = total;
+      ++i;
+      if (total < best) {
+        best = total;
+        pick = cd;
+      }
     }
-    if (i < 8) c->tune_ms[i] = total;
-    ++i;
-    if (total < best) {
-      best = total;
-      pick = cd;
-    }
+    cudaEventDestroy(e0);
+    cudaEventDestroy(e1);
   }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
   c->tuned_Lb = a.Lb;
   c->tuned_col_tile = pick.ct;
   c->tuned_chunk = pick.chunk;
   return CDK_OK;
 }
 
-// Times the Hankel tensor-core x pass on the search's first wave (rotations in the order the
-// waves use) under each candidate shape -- one or two columns per CTA (n <= 64), 1 to 3 K-steps
-// per ring stage, ring caps of 4, 8, 16 and 32 stages -- and keeps the fastest for this ligand box. The candidates run the same
-// MMAs per column in the same order, so the results are identical whichever wins.
+// Times the Hankel tensor-core x pass and the inverse pass that reads its B on the search's first wave (rotations
+// in the order the waves use, the plane kernel before each run as in a search) under each candidate shape --
+// the plan's own first, then one or two columns per CTA (n <= 64), 1 to 3 K-steps per ring stage, ring caps of
+// 4, 8, 16 and 32 stages -- and keeps the fastest for this ligand box, or the plan's own where none is 2 % faster.
+// The inverse pass counts because two columns per CTA give it B in column pairs, which the paired kernels do
+// not read (32^3 split-FP16, K = 3: x pass 0.99 -> 0.93 ms per 2e4 rotations, inverse 0.98 -> 1.79). The candidates
+// run the same MMAs per column in the same order, so the results are identical whichever wins.
 int autotune_hankel(cdk_ctx* c, WaveArgs a, const RotDesc* order, long nRot, int wave, bool f16,
                     const float* osc, cudaStream_t s) {
   a.nrot = (int)std::min<long>(wave, nRot);
   a.rots = order;
   CDK_CUDA(launch_prep(a, s));
-  CDK_CUDA(launch_spread_yz(a, s));
   struct Cand { int cols, nb, ks; };
   std::vector<Cand> cands;
+  {
+    HankelPlan p{};
+    if (hankel_plan(c->n, c->K, a.Lb, f16, c->opts.reserved[5] & 3, &p, 0, (c->opts.reserved[5] >> 2) & 7))
+      cands.push_back({p.cols, p.nb, p.ks});
+  }
   for (int cols : {1, 2})
     for (int ks : {1, 2, 3})
       for (int nb : {4, 8, 16, 32}) {
@@ -251,17 +263,20 @@ int autotune_hankel(cdk_ctx* c, WaveArgs a, const RotDesc* order, long nRot, int
     HankelPlan p{};
     hankel_plan(c->n, c->K, a.Lb, f16, cd.cols, &p, cd.nb, cd.ks);
     hankel_b_layout(p, a);
-    float ms = 0.f, total = 0.f;
-    for (int rep = 0; rep < 2; ++rep) {
+    a.key_slots = a.bpairs ? yz_pairs_key_slots(a) : 0;
+    float ms = 0.f, total = 1e30f;
+    for (int rep = 0; rep < 4; ++rep) {
+      CDK_CUDA(launch_spread_yz(a, s));
       CDK_CUDA(cudaEventRecord(e0, s));
       CDK_CUDA(launch_xpass_hankel(a, c->d_ptilde, osc, p, s));
+      CDK_CUDA(launch_yz_inv_argmin(a, s));
       CDK_CUDA(cudaEventRecord(e1, s));
       CDK_CUDA(cudaEventSynchronize(e1));
       CDK_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-      if (rep == 1) total = ms;  // second run: warm caches
+      if (rep > 0) total = std::min(total, ms);  // after the first: warm caches and clocks
     }
     if (i < 8) c->tune_ms[i] = total;
-    ++i;
+    if (i++ == 0) total *= 0.98f;  // the plan's own
     if (total < best) {
       best = total;
       pick = cd;
@@ -402,8 +417,6 @@ int run_waves(cdk_ctx* c, const float* d_coor, const AtomParam* d_params, const 
     set_error("column tile must be 8 or 16 (n <= 64) or 8 (n > 64)");
     return CDK_ERR_INVALID;
   }
-  CDK_CUDA(cudaMemsetAsync(c->d_misc + 2, 0, 3 * sizeof(unsigned int), s));
-  CDK_CUDA(cudaMemsetAsync(c->d_work, 0, 8 * sizeof(unsigned long long), s));
   const bool umma = tc && !rows && variant != 1 && umma_supported(n, Lb);
   a.work = c->d_work;
   const bool prof = c->opts.reserved[0] != 0;
@@ -460,10 +473,16 @@ int run_waves(cdk_ctx* c, const float* d_coor, const AtomParam* d_params, const 
     hankel_plan(n, K, Lb, f16form, c->tuned_hx_cols, &hp, c->tuned_hx_nb, c->tuned_hx_ks);
   if (hankel) hankel_b_layout(hp, a);
   if (c->opts.reserved[2]) c->tuned_any_Lb = Lb;
+  // after the timing runs, whose errors and work are not the search's
+  CDK_CUDA(cudaMemsetAsync(c->d_misc + 2, 0, 3 * sizeof(unsigned int), s));
+  CDK_CUDA(cudaMemsetAsync(c->d_work, 0, 8 * sizeof(unsigned long long), s));
   for (long r0 = 0; r0 < nRot; r0 += wave) {
     a.nrot = (int)std::min<long>(wave, nRot - r0);
     a.rots = order + r0;
-    if (!tc) xpass_b_layout(a);
+    if (!tc) {
+      xpass_b_layout(a);
+      a.chunk = a.nrot < kTunedFp32Rotations && c->tuned_Lb == Lb ? c->tuned_chunk : 0;
+    }
     a.key_slots = a.bpairs ? yz_pairs_key_slots(a) : 0;
     cudaEvent_t* ev = prof ? &c->kev[(size_t)waves * (kLaunchesPerWave + 1)] : nullptr;
     if (prof) CDK_CUDA(cudaEventRecordWithFlags(ev[0], s, evflags));

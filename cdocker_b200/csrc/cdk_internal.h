@@ -40,12 +40,12 @@ struct AtomParam {
 struct RotRec {
   float mn[3];      // min corner of the rotated ligand (GetMinCoors)
   int W[3];         // translation window per axis: n - int(len/h) - 2
-  int ext[3];       // cells touched by the spread per axis (max cell index + 2)
+  int ext_y;        // cells touched by the spread along y (max cell index + 2)
+  int param_off;    // first AtomParam of its ligand (ConfDesc.param_off)
+  int pad;
   int valid;        // 1 when every window is non-empty
   int err;          // nonzero when the ligand box exceeded the planned box
   int nA;           // atoms
-  int param_off;    // first AtomParam of its ligand (ConfDesc.param_off)
-  int pad[3];
   short xlo[KMAX];  // per channel: first and last x plane touched (xlo > xhi: empty)
   short xhi[KMAX];
   // streamed tensor-core x pass, first record of each 128-rotation tile only: the tile's stage
@@ -53,9 +53,9 @@ struct RotRec {
   // per column), written by k_tile_plan
   unsigned long long tplan[4];
 };
-// the x ranges are read as 16-byte vectors
-static_assert(offsetof(RotRec, xlo) % 16 == 0 && offsetof(RotRec, tplan) % 16 == 0 && sizeof(RotRec) % 16 == 0,
-              "RotRec vector alignment");
+// the x ranges are read as 16-byte vectors; the no-alloc search's limit counts these bytes per rotation
+static_assert(offsetof(RotRec, xlo) % 16 == 0 && offsetof(RotRec, tplan) % 16 == 0 && sizeof(RotRec) == 48 + 4 * KMAX + 32,
+              "RotRec vector alignment and size");
 
 // Everything one wave of rotations needs on the device.
 struct WaveArgs {

@@ -205,8 +205,8 @@ __global__ void __launch_bounds__(128) k_prep(WaveArgs a) {
     for (int d = 0; d < 3; ++d) {
       rec->mn[d] = mn[d];
       rec->W[d] = W[d];
-      rec->ext[d] = s_ext[warp][d];
     }
+    rec->ext_y = s_ext[warp][1];
     rec->valid = (valid && !err) ? 1 : 0;
     rec->err = err;
     rec->nA = nA;
@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(256) k_spread_yz(WaveArgs a) {
   if (x < xlo || x > xhi) return;
   const int tid = threadIdx.x, nthr = blockDim.x;
   for (int i = tid; i < N; i += nthr) tw[i] = a.tw[i];
-  const int npairs = min(N / 2, (rec->ext[1] + 1) / 2);
+  const int npairs = min(N / 2, (rec->ext_y + 1) / 2);
   float* Pf = reinterpret_cast<float*>(P);
   for (int i = tid; i < npairs * (N + 1); i += nthr) P[i] = make_float2(0.f, 0.f);
   __syncthreads();

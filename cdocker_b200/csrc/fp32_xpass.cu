@@ -12,12 +12,14 @@
 // The outputs q and q + 4 differ in one sign before their twiddles, so the two live in one
 // register pair each and most of the arithmetic is packed (pair_fft.cuh).
 //
-// What bounds it: issue slots and the FP32 pipe (at 64^3, box of 21 planes: issue 63 % active, FMA
-// pipe 51 %, per thread and channel about 430 instructions of which 226 floating point and 42 shared
-// loads). Measured on a B200, K = 9, against the radix kernel that exchanged between the stages for
-// every channel (its issue slots went to shared-memory traffic and block barriers): 32^3, 500
-// rotations 0.373 -> 0.145 ms; 64^3, 5,000 rotations 15.1 -> 7.2 ms; 96^3, 999 rotations 10.7 -> 4.2
-// ms; 128^3, 1,000 rotations 26.1 -> 11.1 ms; results bit-identical.
+// What bounds it: latency at one CTA of 16 warps per SM (registers, receptor tile and rings). At 64^3, box
+// of 22 planes, issue is 63 % active, the shared-memory path 67 %, the FMA pipe 50 %; a warp waits, per issue,
+// 1.1 for fixed latencies, 0.8 for shared loads, 0.7 each for the FP32 pipe and the channel's barrier (per
+// thread and channel about 430 instructions, 226 floating point, 42 shared loads). Measured on a B200, K = 9,
+// against k_xpass_block (block_xpass.cu), which exchanges between the stages for every channel and spends its
+// issue slots on shared-memory traffic and block barriers: 32^3, 500 rotations 0.373 -> 0.145 ms; 64^3, 5,000
+// rotations 15.1 -> 7.2 ms; 96^3, 999 rotations 10.7 -> 4.2 ms; 128^3, 1,000 rotations 26.1 -> 11.1 ms; results
+// bit-identical. That kernel takes the waves where it is the faster (xpass_block_stages below).
 //
 // CTA = 8 columns x a chunk of rotations; its 8-column tile of the receptor spectra stays in
 // shared memory. 8 columns and not 16 or 32: the tile fits beside the rings at every n and K <=

@@ -7,9 +7,9 @@
 //                 sums of separable spectra of their trilinear weights -> A; larger ligands, per
 //                 (rotation, channel, x plane): spread the atoms into shared memory (FillLigandGrid's
 //                 arithmetic), then the 2-D real-to-complex FFT   (src/FillLigandGrid.cpp)
-//   xpass         (fp32_xpass.cu) per spectral column tile: FFT along x of every channel, the conjugate
-//                 product with the resident receptor spectra summed over channels, and the
-//                 inverse FFT along x, keeping only the translation window -> B
+//   xpass         (fp32_xpass.cu; block_xpass.cu for a few rotations) per spectral column tile: FFT along x
+//                 of every channel, the conjugate product with the resident receptor spectra summed over
+//                 channels, and the inverse FFT along x, keeping only the translation window -> B
 //                                                       (src/kernel.cu ConjMult + SumGrids)
 //   yz_inv_argmin (yz_pairs.cu) per (rotation, planes x, x + 1 in window): inverse FFT over y, complex-
 //                 to-real over z, min / first argmin over the window, folded into one 64-bit key per
@@ -416,7 +416,8 @@ struct DirectShape {
   static constexpr int NZH = N / 2 + 1, NCOL = N * NZH;
   static constexpr int Q = NCOL / 4;  // column quads: c, c + Q, c + 2 Q, c + 3 Q share kz
   static_assert(NCOL % 4 == 0 && Q % NZH == 0, "a quad's columns share kz");
-  // measured (ms): planes at 64^3, 5,000 rotations: 384 x 2 1.52, 256 x 3 1.65; at 32^3 256 x 3 is the
+  // measured (ms), ligands of 40 atoms (32^3 24, 96^3 80, 128^3 60); shared memory grows with the atoms, and above
+  // about 80 fewer CTAs are resident than asked for. Planes at 64^3, 5,000 rotations: 384 x 2 1.52, 256 x 3 1.65; at 32^3 256 x 3 is the
   // faster; FP16 rows at 64^3, 1e5 rotations: 256 x 3 27.1, 384 x 2 27.7, 192 x 4 27.4; at 128^3, 4,000:
   // 384 x 2 5.6, 256 x 3 6.2 (shared memory holds two CTAs); BF16 rows, 64 result words per thread: at
   // 64^3, 2e4: 192 x 3 9.7, 256 x 2 10.0; at 96^3, 2,000: 2.35 and 2.30; at 128^3, 1,000: 384 x 1 2.5,

@@ -85,3 +85,14 @@ def test_caller_owned_memory_and_graphs():
     with Receptor(grids, 0.5, use_graphs=1) as rec:
         for count in (1, 1, 1, 8, 8, 8, 2, 2, 2):
             same(rec.search(*lig[:4], lig[4][:, :count]), want, count)
+
+
+@pytest.mark.parametrize("n,box", [(32, 9), (64, 40)])
+def test_infinite_receptor(n, box):
+    """A receptor grid that holds an infinity: the same bits from both kernels (NaN energies among them)."""
+    grids, lig = workload(n, 4, box, 40)
+    grids[1, 2, 3, 4] = np.inf
+    with Receptor(grids, 0.5) as rec:
+        want = rec.search(*lig)
+        for count in (1, 3):
+            same(rec.search(*lig[:4], lig[4][:, :count]), want, count)

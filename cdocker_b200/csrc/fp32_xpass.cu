@@ -551,19 +551,19 @@ cudaError_t launch_xp(const WaveArgs& a, const XpPlan& p, cudaStream_t s) {
 }  // namespace
 
 // Waves that k_xpass_block (block_xpass.cu) searches faster, x pass and inverse pass together; k_xpass_pairs is
-// the faster on the other side. Measured, time of the former's over the latter's:
+// the faster on the other side. Measured, time of the former over the latter:
 //   few rotations: a set of four is not full, and the pairs' receptor tile, records and rings take the whole SM
-//     before the first one. Boxes up to n/2, K = 2 to 16: n = 32, 3 rotations 0.89-1.08, 4 0.98-1.20; 64, 5
-//     0.81-0.97, 8 1.0-1.24; 96, 5 0.68-1.02, 8 0.95-1.41; 128, 3 0.77-0.99, 4 0.89-1.23. Larger boxes (eight
-//     inputs per first-stage output): 64, 7 rotations about 0.9, 16 1.16-1.6; 96, 8 0.62-1.03, 16
-//     0.95-1.2 (K >= 10 0.76-1.1, 32 0.9-1.4); 128, 4 0.6-0.9, 16 0.8-1.4.
+//     before the first one. Boxes up to n/2, K = 2 to 16: n = 32, 3 rotations 0.89-1.08, 4 0.98-1.20
+//     (K = 2: 5 0.96-1.0, 6 1.09); 64, 5 0.81-0.97, 8 1.0-1.24; 96, 5 0.68-1.02, 8 0.95-1.41; 128, 3 0.77-0.99,
+//     4 0.89-1.23. Larger boxes (eight inputs per first-stage output): 64, 7 rotations about 0.9, 16
+//     1.16-1.6; 96, 8 0.62-1.03, 16 0.95-1.2 (K >= 10 0.76-1.1, 32 0.9-1.4); 128, 4 0.6-0.9, 16 0.8-1.4.
 //   128^3, boxes far above n/2: beside the receptor tile one group of warps is left per SM. K = 5 to 9, any number of
 //     rotations: boxes of 79 planes 1.04-1.14, 86 0.78-1.04, 95 0.77-0.96, 111 0.56-0.7; K = 12, 16 (the block
 //     kernel at one CTA per SM): 86 1.16-1.44, 95 0.85-1.14, 102 0.83-0.92; K <= 3 (two groups) 1.3-1.5.
 bool xpass_block_stages(const WaveArgs& a) {
   const bool wide = a.Lb > a.n / 2;
   switch (a.n) {
-    case 32: return a.nrot <= 3;
+    case 32: return a.nrot <= (a.K <= 2 ? 5 : 3);
     case 64: return a.nrot <= (wide ? 7 : 5);
     case 96: return a.nrot <= (!wide ? 5 : a.K < 10 ? 15 : 24);
     default: return a.nrot <= (wide ? 8 : 3) || (a.K >= 5 && a.Lb > (a.K < 10 ? 80 : 88));
